@@ -6,18 +6,17 @@
 // (dax::Id = int32, int64, unsigned, dax::Scalar = float) with values of up
 // to 16 bytes (a dax::Vector3 is 12).
 //
-// Tiles: the float scan and the sort work on kPTile elements (256 threads x
-// 16), the integer scan and the compaction on 64 KB of elements:
+// Tiles: the float scan works on kPTile elements (256 threads x 16), the sort
+// on kSortTile, the integer scan and the compaction on 64 KB of elements:
 //   scan     integers: one pass, each tile's prefix found by a decoupled
-//            look-back over the tiles before it; floats (and the sort's
-//            histograms): reduce-then-scan, tile sums, one block scanning
-//            the sums, then each tile scanned with its prefix, whose fixed
-//            order of additions gives the same result on every run (in place
-//            allowed for both);
-//   sort     LSD radix sort, 8-bit digits, stable: per pass a per-tile digit
-//            histogram, a scan of the histograms in digit-major order, and a
-//            scatter that ranks each element among equal digits of its tile
-//            (warp match + per-warp counts) in element order;
+//            look-back over the tiles before it; floats: reduce-then-scan,
+//            tile sums, one block scanning the sums, then each tile scanned
+//            with its prefix, whose fixed order of additions gives the same
+//            result on every run (in place allowed for both);
+//   sort     LSD radix sort, 8-bit digits, stable, one read and one write of
+//            the elements a pass: a tile ranks its keys by ballots, finds the
+//            earlier tiles' digit counts by a look-back, and writes its digits'
+//            runs; up to 8192 elements are sorted in one block;
 //   compact  one pass on the integer scan's machinery: a tile's kept
 //            elements are counted as it lands, its offset found by the
 //            look-back, and the kept elements written at their places
@@ -297,6 +296,9 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
+}
+__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -682,185 +684,448 @@ template <> struct Bits<unsigned long long> {
   static constexpr unsigned long long sign = 0x8000000000000000ull;
 };
 
-template <typename U>
-__device__ __forceinline__ U to_ordered(U x, int kind, bool desc) {
-  // kind: 0 unsigned, 1 signed, 2 float
-  U t = x;
-  if (kind == 1) t = x ^ Bits<U>::sign;
-  if (kind == 2) t = (x & Bits<U>::sign) ? (U)~x : (U)(x ^ Bits<U>::sign);
-  return desc ? (U)~t : t;
-}
-
-template <typename U>
-__device__ __forceinline__ U from_ordered(U t, int kind, bool desc) {
-  if (desc) t = (U)~t;
-  if (kind == 1) return t ^ Bits<U>::sign;
-  if (kind == 2) return (t & Bits<U>::sign) ? (U)(t ^ Bits<U>::sign) : (U)~t;
-  return t;
-}
-
 // The ordering map of a sort pass: keys read from the caller's array are
-// mapped to ordered bits as they are loaded (the first pass, `in`), and
-// mapped back as the last pass stores them (`out`), so that no pass of its
-// own goes over the keys for either.
+// mapped to ordered bits as they are loaded (the first pass), and mapped back
+// as the last pass stores them, so that no pass of its own goes over the keys
+// for either.  Branch-free: x ^ (flip where the sign bit is set) ^ flop, with
+// flip = all bits but the sign for floats, 0 otherwise, and flop = the sign
+// bit for signed and float keys, complemented for descending order; both 0
+// where a pass maps nothing.  flip leaves the sign bit, so the inverse is the
+// same two steps in the other order.
+template <typename U>
 struct KeyOrder {
-  int kind;  // 0 unsigned, 1 signed, 2 float
-  int desc;
-  int in, out;
-  template <typename U>
-  __device__ __forceinline__ U load(U x) const {
-    return in ? to_ordered(x, kind, desc != 0) : x;
+  U in_flip, in_flop, out_flip, out_flop;
+  KeyOrder(int kind, bool desc, bool in, bool out) {
+    const U flip = kind == 2 ? (U)~Bits<U>::sign : (U)0;
+    const U flop = (U)((kind ? Bits<U>::sign : (U)0) ^ (desc ? ~(U)0 : (U)0));
+    in_flip = in ? flip : 0;
+    in_flop = in ? flop : 0;
+    out_flip = out ? flip : 0;
+    out_flop = out ? flop : 0;
   }
-  template <typename U>
+  static __device__ __forceinline__ U sign_mask(U x) {
+    return sizeof(U) == 4 ? (U)((int32_t)x >> 31) : (U)((int64_t)x >> 63);
+  }
+  __device__ __forceinline__ U load(U x) const { return x ^ (sign_mask(x) & in_flip) ^ in_flop; }
   __device__ __forceinline__ U store(U t) const {
-    return out ? from_ordered(t, kind, desc != 0) : t;
+    t ^= out_flop;
+    return t ^ (sign_mask(t) & out_flip);
   }
 };
 
-// Digit histogram of each tile, stored digit-major: hist[d * tiles + tile].
+// One sweep per digit.  A pass reads every key (and value) once and writes it
+// once: a block takes a tile of kSortTile elements from a ticket counter, ranks
+// its keys, publishes its count of every digit, finds how many keys of each
+// digit the earlier tiles hold by looking back over their published counts
+// (thread = digit), and writes the tile out in digit order.  The digits'
+// global starts come from one histogram of all passes' digits, since a pass
+// only permutes the keys.
+//
+// Why this shape (100 M int32 pairs): a pass per tile histogram, scan of the
+// histograms and scatter read the keys twice, and the scatter spent 11.7 of
+// its 17 stall cycles an instruction on __match_any_sync (short scoreboard)
+// and gathered its values from global memory in digit order: 1.31 ms a pass.
+// Here equal digits are found by eight ballots, values pass through shared
+// memory like the keys, and the look-back replaces histogram and scan:
+// 0.51 ms a pass, against 0.24 ms for its 1.6 GB at the copy bandwidth.  What
+// is left is about 93 instructions a row of 32 keys and the random shared
+// memory accesses of counters and places (63 % of that pipe); 16 warps of 16
+// keys a thread (64 registers, two blocks an SM) cannot hide all of both.
+//
+// State of (tile, digit), one 32-bit word, zeroed before the pass: 0 nothing
+// yet; count + 1 (count <= kSortTile) the tile's own count; bit 31 | sum the
+// count over the tiles up to and including it (n < 2^31).
+// Tickets go out in tile order, so a wait is only ever on a block that is
+// running.  The wait is bounded all the same, and a thread whose wait runs out
+// counts the missing tile's digit from the keys themselves (a pass never
+// writes the array it reads), so the result does not depend on it.
+constexpr int kSortThreads = 512;
+constexpr int kSortItems = 16;
+constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr uint32_t kSortInc = 0x80000000u;
+
+int sort_tiles(long long n) { return (int)((n + kSortTile - 1) / kSortTile); }
+
+// Lanes whose digit (bits shift .. shift + 7 of the key) equals this lane's:
+// a ballot per bit.
 template <typename U>
-__global__ void __launch_bounds__(kPT) k_digit_hist(const U* __restrict__ keys, long long n,
-                                                    int shift, uint32_t* __restrict__ hist,
-                                                    int tiles, KeyOrder ord) {
-  __shared__ uint32_t s_h[256];
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    s_h[threadIdx.x] = 0;
-    __syncthreads();
-    const long long b = (long long)tile * kPTile;
-#pragma unroll 4
-    for (int e = 0; e < kPI; ++e) {
-      const long long i = b + e * kPT + threadIdx.x;
-      if (i < n) atomicAdd(&s_h[(unsigned)(ord.load(keys[i]) >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    hist[(long long)threadIdx.x * tiles + tile] = s_h[threadIdx.x];
-    __syncthreads();
+__device__ __forceinline__ unsigned equal_digits(U key, int shift) {
+  const unsigned d = (unsigned)(key >> shift);
+  unsigned peers = kFull;
+#pragma unroll
+  for (int b = 0; b < 8; ++b)
+    asm volatile("{\n .reg .pred p;\n .reg .b32 t, v;\n"
+        " and.b32 t, %1, %2;\n setp.ne.u32 p, t, 0;\n"
+        " vote.sync.ballot.b32 v, p, 0xffffffff;\n"
+        " @!p not.b32 v, v;\n and.b32 %0, %0, v;\n}\n"
+        : "+r"(peers)
+        : "r"(d), "r"(1u << b));
+  return peers;
+}
+
+// Ranks a warp's keys (rows of 32, in row then lane order) among its equal
+// digits; cnt: the warp's 256 counters, zero before, its digit counts after.
+// FULL: every row holds 32 keys; else the first `count` places do.
+template <bool FULL, typename U>
+__device__ __forceinline__ void warp_rank(const U (&key)[kSortItems], uint32_t (&rank)[kSortItems],
+                                          int shift, int count, int lane, uint32_t* cnt) {
+  const unsigned lt = (1u << lane) - 1u;
+  constexpr int kG = 4;  // rows whose masks, which do not depend on one another, come first
+#pragma unroll
+  for (int e0 = 0; e0 < kSortItems; e0 += kG) {
+    unsigned peers[kG];
+#pragma unroll
+    for (int g = 0; g < kG; ++g)
+      if (FULL || 32 * (e0 + g) < count) {
+        peers[g] = equal_digits(key[e0 + g], shift);
+        if (!FULL) peers[g] &= low_mask(count - 32 * (e0 + g));
+      }
+#pragma unroll
+    for (int g = 0; g < kG; ++g)
+      if (FULL || 32 * (e0 + g) < count) {
+        uint32_t* c = cnt + ((unsigned)(key[e0 + g] >> shift) & 255u);
+        const bool ok = FULL || lane < count - 32 * (e0 + g);
+        const unsigned below = __popc(peers[g] & lt);
+        const uint32_t before = ok ? *c : 0u;
+        __syncwarp();
+        if (ok && below == 0u) *c = before + __popc(peers[g]);
+        __syncwarp();
+        rank[e0 + g] = before + below;
+      }
   }
 }
 
-// Stable scatter of one pass.  Warp w of a tile owns its 512 consecutive
-// elements (tile-local w*512 + e*32 + lane, e = 0..15, loads coalesced) and
-// ranks them in element order against warp-private digit counters (warp
-// match: equal digits of earlier lanes, plus the warp's earlier rounds).  A
-// block-wide prefix over (digit, warp) and over the tile's digits then gives
-// every element its place in the tile sorted by digit; keys and source
-// indices are staged there in shared memory, and written out in that order:
-// consecutive threads write consecutive places of one digit's run (the
-// tile's offset for the digit, from the scanned histograms), values gathered
-// from the tile's own range.
-// VW: 32-bit words a value (0 for Sort).  The tile's 16 keys a thread are
-// loaded before any is ranked, and in the write-out each thread gathers its
-// 16 values before storing them: each of those loads is otherwise a DRAM
-// round trip of its own.
-template <typename U, int VW>
-__global__ void __launch_bounds__(kPT) k_digit_scatter(const U* __restrict__ kin,
-                                                       U* __restrict__ kout,
-                                                       const uint32_t* __restrict__ vin,
-                                                       uint32_t* __restrict__ vout,
-                                                       long long n, int shift,
-                                                       const uint32_t* __restrict__ off,
-                                                       int tiles, KeyOrder ord) {
-  extern __shared__ unsigned long long s_dyn[];
-  U* s_key = reinterpret_cast<U*>(s_dyn);                        // [kPTile]
-  uint32_t* s_src = reinterpret_cast<uint32_t*>(s_key + kPTile);  // [kPTile]
-  uint32_t* s_cnt = s_src + kPTile;                               // [kPT/32][256]
-  uint32_t* s_dst = s_cnt + (kPT / 32) * 256;                     // [256] global run start - local start
-  uint32_t* s_warp = s_dst + 256;                                 // [kPT/32]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  uint32_t* cnt = s_cnt + warp * 256;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+// Turns the warps' digit counts s_cnt[warp][256] into each (warp, digit)'s
+// first place in the tile sorted by digit; threads 0..255 return their
+// digit's count and, in *start, its first place.  s_warp: 8 words.
+__device__ __forceinline__ uint32_t place_digits(uint32_t* s_cnt, uint32_t* s_warp, uint32_t* start) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t tot = 0, x = 0;
+  if (tid < 256) {
 #pragma unroll
-    for (int w = 0; w < kPT / 32; ++w) s_cnt[w * 256 + threadIdx.x] = 0;
-    __syncthreads();
-    const long long tb = (long long)tile * kPTile;
-    const int lb = warp * (kPI * 32);
-    U key[kPI];
-    uint32_t rank[kPI];
-#pragma unroll
-    for (int e = 0; e < kPI; ++e) {
-      const long long i = tb + lb + e * 32 + lane;
-      key[e] = i < n ? ord.load(kin[i]) : (U)0;
-    }
-#pragma unroll
-    for (int e = 0; e < kPI; ++e) {
-      const bool ok = tb + lb + e * 32 + lane < n;
-      const unsigned d = ok ? ((unsigned)(key[e] >> shift) & 255u) : 256u;
-      const unsigned peers = __match_any_sync(kFull, d);
-      const uint32_t before = d < 256u ? cnt[d] : 0u;
-      rank[e] = before + __popc(peers & lt);
-      __syncwarp();
-      if (d < 256u && lane == __ffs(peers) - 1) cnt[d] = before + __popc(peers);
-      __syncwarp();
-    }
-    __syncthreads();
-    // thread t = digit: its tile count, prefix over warps, and the tile-local
-    // start of its run (exclusive scan over the digits)
-    uint32_t tot = 0;
-#pragma unroll
-    for (int w = 0; w < kPT / 32; ++w) {
-      const uint32_t c = s_cnt[w * 256 + threadIdx.x];
-      s_cnt[w * 256 + threadIdx.x] = tot;
+    for (int w = 0; w < kSortWarps; ++w) {
+      const uint32_t c = s_cnt[w * 256 + tid];
+      s_cnt[w * 256 + tid] = tot;
       tot += c;
     }
-    uint32_t x = tot;
+    x = tot;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t y = __shfl_up_sync(kFull, x, d);
       if (lane >= d) x += y;
     }
     if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    uint32_t lstart = x - tot;
-    for (int w = 0; w < warp; ++w) lstart += s_warp[w];
-#pragma unroll
-    for (int w = 0; w < kPT / 32; ++w) s_cnt[w * 256 + threadIdx.x] += lstart;
-    s_dst[threadIdx.x] = off[(long long)threadIdx.x * tiles + tile] - lstart;
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < kPI; ++e) {
-      const int li = lb + e * 32 + lane;
-      if (tb + li < n) {
-        const unsigned d = (unsigned)(key[e] >> shift) & 255u;
-        const uint32_t lp = cnt[d] + rank[e];
-        s_key[lp] = key[e];
-        s_src[lp] = (uint32_t)li;
-      }
-    }
-    __syncthreads();
-    const int valid = (int)min((long long)kPTile, n - tb);
-    constexpr int kJ = kPTile / kPT;
-    constexpr int kV = VW > 0 ? VW : 1;
-    uint32_t at[kJ], v[kJ][kV];
-#pragma unroll
-    for (int jj = 0; jj < kJ; ++jj) {
-      const int j = threadIdx.x + jj * kPT;
-      if (j < valid) {
-        const U k = s_key[j];
-        at[jj] = s_dst[(unsigned)(k >> shift) & 255u] + j;
-        kout[at[jj]] = ord.store(k);
-        if constexpr (VW > 0) {
-          const long long src = tb + s_src[j];
-#pragma unroll
-          for (int q = 0; q < VW; ++q) v[jj][q] = vin[src * VW + q];
-        }
-      }
-    }
-    if constexpr (VW > 0) {
-#pragma unroll
-      for (int jj = 0; jj < kJ; ++jj)
-        if (threadIdx.x + jj * kPT < valid)
-#pragma unroll
-          for (int q = 0; q < VW; ++q) vout[(long long)at[jj] * VW + q] = v[jj][q];
-    }
-    __syncthreads();
   }
+  __syncthreads();
+  if (tid < 256) {
+    x -= tot;
+    for (int w = 0; w < warp; ++w) x += s_warp[w];
+    *start = x;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) s_cnt[w * 256 + tid] += x;
+  }
+  return tot;
+}
+
+// Digit counts of all keys for `npass` passes from digit `first`:
+// hist[p * 256 + digit], zero before.  Bound by the shared-memory atomics,
+// about eight lanes a cycle whether or not they collide (100 M int32 keys, four
+// digits: 177 us; sixteen copies of every counter measured the same).
+template <typename U>
+__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const U* __restrict__ keys, long long n,
+                                                             int first, int npass,
+                                                             uint32_t* __restrict__ hist,
+                                                             KeyOrder<U> ord) {
+  constexpr int kD = (int)sizeof(U);
+  __shared__ uint32_t s_h[kD * 256];
+  for (int i = threadIdx.x; i < kD * 256; i += kSortThreads) s_h[i] = 0;
+  __syncthreads();
+  const long long stride = (long long)gridDim.x * kSortThreads;
+  for (long long i = (long long)blockIdx.x * kSortThreads + threadIdx.x; i < n; i += 4 * stride) {
+    U k[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) k[u] = i + u * stride < n ? keys[i + u * stride] : (U)0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * stride < n) {
+        const U x = ord.load(k[u]) >> (8 * first);
+#pragma unroll
+        for (int p = 0; p < kD; ++p)
+          if (p < npass) atomicAdd(&s_h[p * 256 + ((unsigned)(x >> (8 * p)) & 255u)], 1u);
+      }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < npass * 256; i += kSortThreads)
+    if (s_h[i]) atomicAdd(hist + i, s_h[i]);
+}
+
+// Shared memory above 48 KB is opted into once per device and kernel; a
+// failure shows as the launch's error.
+void opt_in_smem(const void* kernel, size_t smem, int* done) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || done[dev]) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+      cudaSuccess)
+    done[dev] = 1;
+}
+
+// Keys of `tile` whose digit is d, counted from the keys (a wait ran out).
+template <typename U>
+__device__ __forceinline__ uint32_t count_digit(const U* kin, long long n, int tile, int shift,
+                                             unsigned d, KeyOrder<U> ord) {
+  const long long b = (long long)tile * kSortTile;
+  const long long e = b + kSortTile < n ? b + kSortTile : n;
+  uint32_t c = 0;
+#pragma unroll 1
+  for (long long i = b; i < e; ++i) c += ((unsigned)(ord.load(kin[i]) >> shift) & 255u) == d;
+  return c;
+}
+
+// Keys of digit d in the tiles before `tile`.  kLook states are read at a time.
+constexpr int kLook = 4;
+
+template <typename U>
+__device__ __forceinline__ uint32_t digit_look_back(const uint32_t* state, int tile, unsigned d,
+                                                    const U* kin, long long n, int shift,
+                                                    const KeyOrder<U>& ord) {
+  uint32_t prefix = 0;
+  int t = tile - 1;
+  Spin spin;
+  while (t >= 0) {
+    uint32_t v[kLook];
+#pragma unroll
+    for (int q = 0; q < kLook; ++q)
+      v[q] = t >= q ? ld_relaxed(state + (long long)(t - q) * 256 + d) : kSortInc;
+    bool waiting = false;
+#pragma unroll
+    for (int q = 0; q < kLook; ++q) {
+      if (t < 0 || waiting) continue;
+      if (v[q] & kSortInc) {
+        prefix += v[q] & ~kSortInc;
+        t = -1;
+      } else if (v[q]) {
+        prefix += v[q] - 1u;
+        --t;
+      } else {
+        waiting = true;
+      }
+    }
+    if (waiting && !spin.more()) {
+      prefix += count_digit(kin, n, t, shift, d, ord);
+      --t;
+    }
+  }
+  return prefix;
 }
 
 template <typename U>
-size_t scatter_smem() {
-  return (size_t)kPTile * sizeof(U) + (size_t)kPTile * 4 + (kPT / 32) * 256 * 4 + 256 * 4 +
-         (kPT / 32) * 4;
+constexpr size_t sweep_smem(int vwords) {
+  return (size_t)kSortTile * sizeof(U) + (vwords ? (size_t)kSortTile * 4 : 0) +
+         (size_t)kSortWarps * 256 * 4 + 256 * 4 + 16 * 4;
+}
+
+// One tile of a pass.  VW: 32-bit words a value (0: keys only); FULL: the
+// tile holds kSortTile elements.
+template <typename U, int VW, bool FULL>
+__device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restrict__ kout,
+                                           const uint32_t* __restrict__ vin,
+                                           uint32_t* __restrict__ vout, long long n, int shift,
+                                           const uint32_t* __restrict__ hist,
+                                           uint32_t* __restrict__ state, int tile,
+                                           const KeyOrder<U>& ord, U* s_key, uint32_t* s_val,
+                                           uint32_t* s_cnt, uint32_t* s_dst, uint32_t* s_warp) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long tb = (long long)tile * kSortTile;
+  const int valid = FULL ? kSortTile : (int)(n - tb);
+  const int l0 = warp * (kSortItems * 32) + lane;  // the thread's first element of the tile
+  const U* kt = kin + tb + l0;
+  U key[kSortItems];
+  uint32_t rank[kSortItems];
+#pragma unroll
+  for (int e = 0; e < kSortItems; ++e)
+    key[e] = FULL || l0 + 32 * e < valid ? __ldcs(kt + 32 * e) : (U)0;
+#pragma unroll
+  for (int e = 0; e < kSortItems; ++e) key[e] = ord.load(key[e]);
+  uint32_t* cnt = s_cnt + warp * 256;
+  warp_rank<FULL>(key, rank, shift, valid - (l0 - lane), lane, cnt);
+  __syncthreads();
+  uint32_t lstart = 0;
+  const uint32_t tot = place_digits(s_cnt, s_warp, &lstart);
+  uint32_t* mine = state + (long long)tile * 256 + tid;
+  if (tid < 256) st_relaxed(mine, tile == 0 ? kSortInc | tot : tot + 1u);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < kSortItems; ++e)
+    if (FULL || l0 + 32 * e < valid) {
+      rank[e] += cnt[(unsigned)(key[e] >> shift) & 255u];  // its place in the tile
+      s_key[rank[e]] = key[e];
+    }
+  uint32_t v[VW ? kSortItems : 1];
+  auto load_values = [&](int q) {
+    const uint32_t* vt = vin + (tb + l0) * VW + q;
+#pragma unroll
+    for (int e = 0; e < kSortItems; ++e)
+      if (FULL || l0 + 32 * e < valid) v[e] = VW == 1 ? __ldcs(vt + 32 * e) : vt[32 * e * VW];
+  };
+  auto place_values = [&]() {
+#pragma unroll
+    for (int e = 0; e < kSortItems; ++e)
+      if (FULL || l0 + 32 * e < valid) s_val[rank[e]] = v[e];
+  };
+  if constexpr (VW > 0) load_values(0);  // in flight during the look-back
+  if (tid < 256) {
+    // the digit's start over all keys: an exclusive scan of the 256 counts
+    const uint32_t h = hist[tid];
+    uint32_t x = h;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) s_warp[8 + warp] = x;
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // the 256 digit threads
+    x -= h;
+    for (int w = 0; w < warp; ++w) x += s_warp[8 + w];
+    const uint32_t before = digit_look_back(state, tile, (unsigned)tid, kin, n, shift, ord);
+    if (tile > 0) st_relaxed(mine, kSortInc | (before + tot));
+    s_dst[tid] = x + before - lstart;
+  }
+  if constexpr (VW > 0) place_values();
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < kSortItems; ++e) {
+    const int j = tid + e * kSortThreads;
+    if (FULL || j < valid) {
+      const U k = s_key[j];
+      const uint32_t at = s_dst[(unsigned)(k >> shift) & 255u] + j;
+      kout[at] = ord.store(k);
+      if constexpr (VW > 0) vout[(long long)at * VW] = s_val[j];
+    }
+  }
+  if constexpr (VW > 1) {
+#pragma unroll 1
+    for (int q = 1; q < VW; ++q) {
+      load_values(q);
+      __syncthreads();  // the previous word has left
+      place_values();
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < kSortItems; ++e) {
+        const int j = tid + e * kSortThreads;
+        if (FULL || j < valid) {
+          const uint32_t at = s_dst[(unsigned)(s_key[j] >> shift) & 255u] + j;
+          vout[(long long)at * VW + q] = s_val[j];
+        }
+      }
+    }
+  }
+}
+
+// One pass: hist: the digits' counts over all keys.
+template <typename U, int VW>
+__global__ void __launch_bounds__(kSortThreads, 2)
+    k_radix_sweep(const U* __restrict__ kin, U* __restrict__ kout, const uint32_t* __restrict__ vin,
+                  uint32_t* __restrict__ vout, long long n, int shift,
+                  const uint32_t* __restrict__ hist, uint32_t* __restrict__ state,
+                  unsigned* __restrict__ ticket, KeyOrder<U> ord) {
+  extern __shared__ unsigned long long s_dyn[];
+  U* s_key = reinterpret_cast<U*>(s_dyn);                            // [kSortTile]
+  uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + kSortTile);  // [kSortTile] if VW
+  uint32_t* s_cnt = s_val + (VW ? kSortTile : 0);                    // [kSortWarps][256]
+  uint32_t* s_dst = s_cnt + kSortWarps * 256;  // [256] global place of the run - its local start
+  uint32_t* s_warp = s_dst + 256;              // [16]
+  __shared__ int s_tile;
+  if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
+  for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads) s_cnt[i] = 0;
+  __syncthreads();
+  const int tile = s_tile;
+  if ((long long)tile * kSortTile >= n) return;
+  if ((long long)(tile + 1) * kSortTile <= n)
+    sweep_tile<U, VW, true>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, s_key, s_val,
+                            s_cnt, s_dst, s_warp);
+  else
+    sweep_tile<U, VW, false>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, s_key, s_val,
+                             s_cnt, s_dst, s_warp);
+}
+
+// At most kSortTile elements: every pass in one block's shared memory, the
+// elements' first places carried beside the keys; the values are moved once,
+// at the end (each word of every row is read before any is written).
+template <typename U>
+constexpr size_t block_sort_smem() {
+  return (size_t)kSortTile * (sizeof(U) + 2) + (size_t)kSortWarps * 256 * 4 + 16 * 4;
+}
+
+template <typename U>
+__global__ void __launch_bounds__(kSortThreads, 1)
+    k_sort_block(U* keys, uint32_t* vals, int vwords, int n, int passes, KeyOrder<U> ord) {
+  extern __shared__ unsigned long long s_dyn[];
+  U* s_key = reinterpret_cast<U*>(s_dyn);                            // [kSortTile]
+  uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_key + kSortTile);  // [kSortWarps][256]
+  uint32_t* s_warp = s_cnt + kSortWarps * 256;                       // [8]
+  uint16_t* s_src = reinterpret_cast<uint16_t*>(s_warp + 16);        // [kSortTile]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rows = (n + kSortThreads - 1) / kSortThreads;  // rows of 32 a warp
+  const int w0 = warp * rows * 32;
+  const int count = min(n - w0, rows * 32);  // the warp's keys (<= 0: none)
+  uint32_t* cnt = s_cnt + warp * 256;
+  U key[kSortItems];
+  uint32_t rank[kSortItems];
+  uint16_t src[kSortItems];
+#pragma unroll
+  for (int e = 0; e < kSortItems; ++e) {
+    const int li = w0 + 32 * e + lane;
+    if (e < rows && li < n) {
+      key[e] = ord.load(keys[li]);
+      src[e] = (uint16_t)li;
+    }
+  }
+  for (int p = 0; p < passes; ++p) {
+    const int shift = 8 * p;
+    if (p > 0) {
+#pragma unroll
+      for (int e = 0; e < kSortItems; ++e) {
+        const int li = w0 + 32 * e + lane;
+        if (e < rows && li < n) {
+          key[e] = s_key[li];
+          src[e] = s_src[li];
+        }
+      }
+    }
+    for (int i = tid; i < kSortWarps * 256; i += kSortThreads) s_cnt[i] = 0;
+    __syncthreads();
+    warp_rank<false>(key, rank, shift, count, lane, cnt);
+    __syncthreads();
+    uint32_t start;
+    place_digits(s_cnt, s_warp, &start);
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < kSortItems; ++e) {
+      if (e < rows && w0 + 32 * e + lane < n) {
+        const uint32_t at = cnt[(unsigned)(key[e] >> shift) & 255u] + rank[e];
+        s_key[at] = key[e];
+        s_src[at] = src[e];
+      }
+    }
+    __syncthreads();
+  }
+  for (int j = tid; j < n; j += kSortThreads) keys[j] = ord.store(s_key[j]);
+  for (int q = 0; q < vwords; ++q) {
+    uint32_t v[kSortItems];
+#pragma unroll
+    for (int e = 0; e < kSortItems; ++e) {
+      const int j = tid + e * kSortThreads;
+      if (j < n) v[e] = vals[(int)s_src[j] * vwords + q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < kSortItems; ++e) {
+      const int j = tid + e * kSortThreads;
+      if (j < n) vals[j * vwords + q] = v[e];
+    }
+  }
 }
 
 // ---- single-pass compaction ------------------------------------------------
@@ -1061,42 +1326,69 @@ SortLayout sort_layout(long long n, int key_bytes, int value_bytes) {
   return L;
 }
 
+template <typename U, int VW>
+void launch_sweep(const U* kin, U* kout, const uint32_t* vin, uint32_t* vout, long long n, int shift,
+                  const uint32_t* hist, uint32_t* state, unsigned* ticket, KeyOrder<U> ord,
+                  cudaStream_t s) {
+  static int opted[64] = {};
+  constexpr size_t smem = sweep_smem<U>(VW);
+  opt_in_smem((const void*)k_radix_sweep<U, VW>, smem, opted);
+  k_radix_sweep<U, VW><<<sort_tiles(n), kSortThreads, smem, s>>>(kin, kout, vin, vout, n, shift,
+                                                                hist, state, ticket, ord);
+}
+
 // passes: 8-bit digits to sort, least significant first (an even count, so
 // the result ends in keys/vals); plain = the keys are unsigned, ascending and
 // need no order mapping.
+//
+// Up to kSortTile elements are one launch of one block.  Longer arrays keep
+// the tile states, the digit counts and the tickets in the scratch's
+// histogram section: 1 KB per 4096 elements, of which the states take 1 KB
+// per kSortTile = 8192; the counts of as many passes as fit beside them
+// (all, from 64 K elements) are taken at a time.
 template <typename U>
 void radix_sort(U* keys, uint32_t* vals, int vwords, long long n, int kind, bool desc,
                 char* scratch, int num_sms, cudaStream_t s, int passes = (int)sizeof(U),
                 bool plain = false) {
+  if (n <= kSortTile) {
+    static int opted[64] = {};
+    const KeyOrder<U> ord{kind, desc, !plain, !plain};
+    opt_in_smem((const void*)k_sort_block<U>, block_sort_smem<U>(), opted);
+    k_sort_block<U><<<1, kSortThreads, block_sort_smem<U>(), s>>>(keys, vals, vwords, (int)n, passes,
+                                                                 ord);
+    return;
+  }
   const SortLayout L = sort_layout(n, (int)sizeof(U), 4 * vwords);
   U* ktmp = reinterpret_cast<U*>(scratch + L.ktmp);
   uint32_t* vtmp = reinterpret_cast<uint32_t*>(scratch + L.vtmp);
-  uint32_t* hist = reinterpret_cast<uint32_t*>(scratch + L.hist);
-  void* sums = scratch + L.sums;
-  const int tiles = ptiles(n);
-  const int bh = resident((const void*)k_digit_hist<U>, kPT, num_sms, tiles);
-  const size_t sm = scatter_smem<U>();
-  const void* scat = vwords == 0   ? (const void*)k_digit_scatter<U, 0>
-                     : vwords == 1 ? (const void*)k_digit_scatter<U, 1>
-                     : vwords == 2 ? (const void*)k_digit_scatter<U, 2>
-                     : vwords == 3 ? (const void*)k_digit_scatter<U, 3>
-                                   : (const void*)k_digit_scatter<U, 4>;
-  cudaFuncSetAttribute(scat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  int per = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scat, kPT, sm) != cudaSuccess || per < 1)
-    per = 1;
-  const int bs = (int)(tiles < (long long)num_sms * per ? tiles : (long long)num_sms * per);
+  const int tiles = sort_tiles(n), spare = ptiles(n) - tiles;  // KB beside the states
+  const int group = spare < passes ? spare : passes;           // >= 1 for n > kSortTile
+  // ... [counts of `group` passes][states][ticket], the ticket where L.sums begins
+  uint32_t* state = reinterpret_cast<uint32_t*>(scratch + L.hist) + 256ll * spare;
+  uint32_t* hist = state - 256ll * group;
+  unsigned* ticket = reinterpret_cast<unsigned*>(scratch + L.sums);
+  const int bh = resident_blocks(k_radix_hist<U>, kSortThreads, 0, num_sms,
+                                 (n + 4 * kSortThreads - 1) / (4 * kSortThreads));
   for (int p = 0; p < passes; ++p) {
     const U* ksrc = (p & 1) ? ktmp : keys;
     U* kdst = (p & 1) ? keys : ktmp;
     const uint32_t* vsrc = (p & 1) ? vtmp : vals;
     uint32_t* vdst = (p & 1) ? vals : vtmp;
-    KeyOrder ord{kind, desc ? 1 : 0, !plain && p == 0, !plain && p == passes - 1};
-    k_digit_hist<U><<<bh, kPT, 0, s>>>(ksrc, n, 8 * p, hist, tiles, ord);
-    scan_t<uint32_t>(hist, hist, 256ll * tiles, true, sums, nullptr, num_sms, s);
-    int shift = 8 * p;
-    void* args[] = {&ksrc, &kdst, &vsrc, &vdst, &n, &shift, &hist, const_cast<int*>(&tiles), &ord};
-    cudaLaunchKernel(scat, dim3(bs), dim3(kPT), args, sm, s);
+    const KeyOrder<U> ord{kind, desc, !plain && p == 0, !plain && p == passes - 1};
+    const int at = p % group;
+    // the states and the ticket, and before a group of passes its digit counts
+    uint32_t* clear = at == 0 ? hist : state;
+    cudaMemsetAsync(clear, 0, (size_t)((char*)(ticket + 1) - (char*)clear), s);
+    const int counted = passes - p < group ? passes - p : group;
+    if (at == 0) k_radix_hist<U><<<bh, kSortThreads, 0, s>>>(ksrc, n, p, counted, hist, ord);
+    const uint32_t* h = hist + 256 * at;
+    switch (vwords) {
+      case 0: launch_sweep<U, 0>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+      case 1: launch_sweep<U, 1>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+      case 2: launch_sweep<U, 2>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+      case 3: launch_sweep<U, 3>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+      default: launch_sweep<U, 4>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+    }
   }
 }
 

@@ -272,6 +272,27 @@ def test_sort_by_key_random(A, gb300, n, dtype, vcols, desc):
         assert np.array_equal(vals.cpu().numpy(), ref)
 
 
+# one block's largest sort, the first two-tile sorts, the sizes at which the digit counts of 4 and of 8 passes first
+# fit the scratch at once, ragged last tiles
+@pytest.mark.parametrize("n", [33, 513, 8191, 8192, 8193, 12289, 16384, 16385, 32769, 57345, 65537, 1_000_003])
+@pytest.mark.parametrize("dtype,vcols", [(np.int32, 1), (np.int64, 2), (np.float32, 3), (np.int64, 0)])
+def test_sort_tile_edges(A, gb300, n, dtype, vcols):
+    rng = np.random.default_rng(n)
+    if dtype == np.float32:
+        k = rng.standard_normal(n).astype(np.float32)
+    else:
+        info = np.iinfo(dtype)
+        k = rng.integers(info.min, info.max, n, dtype=dtype)
+    k[: n // 2] = k[rng.integers(0, n // 2 + 1, n // 2)]  # ties: the order of equal keys shows
+    v = np.arange(n * max(vcols, 1), dtype=np.int32).reshape(n, max(vcols, 1))
+    keys, vals = cuda(k), cuda(v) if vcols else None
+    A.SortByKey(keys, vals)
+    order = _stable_order(k, False)
+    assert np.array_equal(keys.cpu().numpy(), k[order])
+    if vcols:
+        assert np.array_equal(vals.cpu().numpy(), v[order])
+
+
 def test_sort_special_inputs(A, gb300):
     for x in (np.zeros(5000, np.int32), np.arange(5000, dtype=np.int32)[::-1].copy(),
               np.arange(5000, dtype=np.int32), np.array([2 ** 31 - 1, -2 ** 31, 0, -1, 1], np.int32)):
