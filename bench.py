@@ -1189,7 +1189,7 @@ def main():
         "config": dict(config_dict(n), frames_in_flight=1, slabs=slab_count,
                        call="dax_gb300_mc_pipeline (count + merged generate, slab-pipelined)",
                        count_pass="fused classify + count launch, then the scan" if args.fused
-                       else "classification, staged count and scan launches",
+                       else "classification, count and scan launches",
                        replay="CUDA graph of the frame's call, captured once" if graph is not None
                        else "direct call per frame"),
         "frames": {"pipelined_direct_calls_ms": ms_direct,

@@ -314,9 +314,9 @@ struct dax_gb300_mc_batch {
   size_t off_goff = 0;
   McLayout L;
   // tuned by dax_gb300_mc_batch_autotune (or set): active words per emit
-  // warp batch, and the dealt (1) or per-lane (0) count pass
+  // warp batch
   int emit_batch = daxgb::kEmitBatch;
-  int dealt = 1;
+  int dealt = 1;  // kept for get_config: there is one count pass
   // grid-set CellGradient and adjoint: totals of the concatenated per-cell
   // and per-point arrays, and per grid the first block of each set launch
   // (d_blk: [gradient][adjoint gradient term][adjoint vertex term], count + 1
@@ -1211,7 +1211,7 @@ int dax_gb300_mc_batch_count(dax_gb300_mc_batch* b, void* d_scratch, size_t scra
   int st = check_launch("batch classify kernel");
   if (st) return st;
   const daxgb::WordOffsets o = b->L.offsets(d_scratch);
-  daxgb::launch_mc_scan(S, bits, o, at<Info>(d_scratch, 0), num_sms(), s, b->dealt);
+  daxgb::launch_mc_scan(S, bits, o, at<Info>(d_scratch, 0), num_sms(), s);
   if ((st = check_launch("batch count/scan kernels"))) return st;
   daxgb::launch_grid_offsets(S, b->L.offsets(d_scratch), at<long long>(d_scratch, b->off_goff), s);
   return check_launch("batch offsets kernel");
@@ -1314,13 +1314,12 @@ int dax_gb300_mc_batch_autotune(dax_gb300_mc_batch* b, int merge, void* d_scratc
   for (int c = b->count; c > 1; c >>= 1) ++lc;
   const long long key = ((long long)lc << 16) | ((long long)lg << 1) | (merge != 0);
   static std::mutex m;
-  static std::map<long long, std::pair<int, int>> cache;
+  static std::map<long long, int> cache;
   {
     std::lock_guard<std::mutex> lock(m);
     auto it = cache.find(key);
     if (it != cache.end()) {
-      b->emit_batch = it->second.first;
-      b->dealt = it->second.second;
+      b->emit_batch = it->second;
       if (h_best_ms) *h_best_ms = -1.0f;  // taken from the cache, not timed
       return DAX_GB300_SUCCESS;
     }
@@ -1331,42 +1330,38 @@ int dax_gb300_mc_batch_autotune(dax_gb300_mc_batch* b, int merge, void* d_scratc
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   if (e != cudaSuccess) return cuda_fail(e, "autotune events");
   float best = 1e30f;
-  int best_batch = b->emit_batch, best_dealt = b->dealt, st = DAX_GB300_SUCCESS;
+  int best_batch = b->emit_batch, st = DAX_GB300_SUCCESS;
   const int batches[3] = {8, 16, 32};
-  for (int d = (b->count > 1 ? 1 : 0); d >= 0 && !st; --d)
-    for (int bi = 0; bi < 3 && !st; ++bi) {
-      b->emit_batch = batches[bi];
-      b->dealt = d;
-      float total = 0.0f;
-      for (int rep = 0; rep < 4 && !st; ++rep) {  // the first run warms up
-        e = cudaEventRecord(e0, s);
-        st = e == cudaSuccess ? dax_gb300_mc_batch_count(b, d_scratch, scratch_bytes, s)
-                              : cuda_fail(e, "autotune");
-        if (!st)
-          st = dax_gb300_mc_batch_generate(b, merge, d_scratch, scratch_bytes, d_verts,
-                                           vert_capacity, d_conn, tri_capacity, s);
-        if (!st) e = cudaEventRecord(e1, s);
-        if (!st && e == cudaSuccess) e = cudaEventSynchronize(e1);
-        float ms = 0.0f;
-        if (!st && e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        if (!st && e != cudaSuccess) st = cuda_fail(e, "autotune timing");
-        if (!st && rep > 0) total += ms;
-      }
-      if (!st) st = read_totals(d_scratch, nullptr, nullptr, s);
-      if (!st && total / 3 < best) {
-        best = total / 3;
-        best_batch = batches[bi];
-        best_dealt = d;
-      }
+  for (int bi = 0; bi < 3 && !st; ++bi) {
+    b->emit_batch = batches[bi];
+    float total = 0.0f;
+    for (int rep = 0; rep < 4 && !st; ++rep) {  // the first run warms up
+      e = cudaEventRecord(e0, s);
+      st = e == cudaSuccess ? dax_gb300_mc_batch_count(b, d_scratch, scratch_bytes, s)
+                            : cuda_fail(e, "autotune");
+      if (!st)
+        st = dax_gb300_mc_batch_generate(b, merge, d_scratch, scratch_bytes, d_verts,
+                                         vert_capacity, d_conn, tri_capacity, s);
+      if (!st) e = cudaEventRecord(e1, s);
+      if (!st && e == cudaSuccess) e = cudaEventSynchronize(e1);
+      float ms = 0.0f;
+      if (!st && e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+      if (!st && e != cudaSuccess) st = cuda_fail(e, "autotune timing");
+      if (!st && rep > 0) total += ms;
     }
+    if (!st) st = read_totals(d_scratch, nullptr, nullptr, s);
+    if (!st && total / 3 < best) {
+      best = total / 3;
+      best_batch = batches[bi];
+    }
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   b->emit_batch = best_batch;
-  b->dealt = best_dealt;
   if (st) return st;
   {
     std::lock_guard<std::mutex> lock(m);
-    cache[key] = std::make_pair(best_batch, best_dealt);
+    cache[key] = best_batch;
   }
   if (h_best_ms) *h_best_ms = best;
   return DAX_GB300_SUCCESS;

@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(256) k_classify_bits(GridSet S, uint32_t* __re
   pdl_trigger();  // the count pass may launch into the SMs this grid frees
   if (init && blockIdx.x == 0 && threadIdx.x == 0) {
     init->error = 0;
-    init->aborted = 0;
     init->ticket = 0;
     init->done = 0;
   }

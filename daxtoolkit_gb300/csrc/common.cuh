@@ -173,9 +173,7 @@ struct Info {
   int error;              // kErr* bits raised on the device
   unsigned ticket;        // next batch of active words for the MC emit warps
   unsigned done;          // MC emit blocks finished (the last resets both)
-  int aborted;            // a count kernel's bounded wait ran out (the scan
-                          //   reports it as kErrTimeout); cleared with error
-  int pad[6];
+  int pad[7];
 };
 
 constexpr int kErrCapacity = 2;    // output buffer too small

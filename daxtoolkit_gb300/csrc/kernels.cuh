@@ -186,19 +186,9 @@ int fused_unit_stages();
 void launch_word_scan(long long rowwords, const uint32_t* wc, const uint32_t* tile_tot,
                       uint32_t* wt, uint32_t* wv, uint32_t* act, Info* info, cudaStream_t s,
                       const uint32_t* abort = nullptr);
-// Marching-cubes K2a of one grid with each scan tile's bits staged in
-// shared memory by bulk TMA copies (staged.cu): k_mc_count's outputs, bit
-// for bit.  False (nothing launched) when a tile's ranges do not fit the
-// shared memory.  A copy that does not arrive sets info->aborted, which the
-// scan reports as kErrTimeout.
-bool launch_mc_count_staged(const Grid& g, const uint32_t* bits, long long nwords,
-                            const WordOffsets& o, Info* info, int num_sms, cudaStream_t s);
 // Marching cubes K2a (counts: triangles, crossing edges) + K2b.
-// dealt != 0: for a grid set, the count pass that deals a warp's active cells
-// to its lanes (the default); 0: the per-lane count pass.  One grid always
-// takes the per-lane pass.
 void launch_mc_scan(const GridSet& S, const uint32_t* bits, const WordOffsets& o, Info* info,
-                    int num_sms, cudaStream_t s, int dealt = -1);
+                    int num_sms, cudaStream_t s);
 void launch_mc_emit(const GridSet& S, bool merge, const uint32_t* bits, const WordOffsets& o,
                     Info* info, float* verts, long long vcap, int32_t* conn, long long tcap,
                     int32_t* ra, int32_t* rb, float* rw, int num_sms, cudaStream_t s);

@@ -98,113 +98,206 @@ __device__ __forceinline__ int nth_bit(uint32_t u, int n) {
   return p;
 }
 
-constexpr int kCountWords = 4;  // consecutive row words per count group
+constexpr int kCountThreads = 512;
+constexpr int kCountSegments = 4;  // grids in a tile that its block takes one after another
 
-// K2a: one 256-thread block per tile of kScanTile row words (grid-stride
-// over tiles).  Thread t counts the 4-word groups t + 256 e (e = 0..3) of
-// the tile, so a warp's groups are consecutive; the block then writes the
-// tile's totals (triangles, crossing edges, active words) to
-// tile_tot[0 / 1 / 2][tile] for the scan.
-__global__ void __launch_bounds__(256) k_mc_count(GridSet S, const uint32_t* __restrict__ bits,
-                                                  uint32_t* __restrict__ wc,
-                                                  uint32_t* __restrict__ tile_tot, int tiles,
-                                                  int tile_begin, int tile_end) {
+// Appends the tile's word `id` (its place in the tile) to the block's list
+// where `on`; every lane of the warp calls it.
+__device__ __forceinline__ void push_word(bool on, int id, unsigned short* list, int* count,
+                                          int lane) {
+  const unsigned b = __ballot_sync(kFull, on);
+  if (!b) return;
+  int at = 0;
+  if (lane == 0) at = atomicAdd(count, __popc(b));
+  at = __shfl_sync(kFull, at, 0) + __popc(b & ((1u << lane) - 1u));
+  if (on) list[at] = (unsigned short)id;
+}
+
+// Whether word lw of grid g may have a crossing edge or an active cell.
+__device__ __forceinline__ bool word_differs(const Grid& g, const uint32_t* __restrict__ bits,
+                                             unsigned lw) {
+  int m;
+  const unsigned r = split_word(g, lw, m);
+  const WordBits wb = load_word_bits(g, bits, r, m);
+  uint32_t diff = wb.w.a ^ wb.w.a1;
+  if (wb.hy) diff |= (wb.w.a ^ wb.w.b) | (wb.w.a ^ wb.w.b1);
+  if (wb.hz) diff |= (wb.w.a ^ wb.w.c) | (wb.w.a ^ wb.w.c1);
+  if (wb.hy && wb.hz) diff |= (wb.w.a ^ wb.w.d) | (wb.w.a ^ wb.w.d1);
+  return (diff & wb.pmask) != 0;
+}
+
+// Lists the words [lo, hi) of grid g, whose bits start at `bits`, that may
+// have a crossing edge or an active cell; word lo is the tile's word id0.
+// A lane walks down one word column over `depth` consecutive rows, so that it
+// combines each row (its words and their +x neighbours, here and one plane
+// up) once, for the row itself and as the next row of the one before.
+// Consecutive lanes take consecutive words; a grid has fewer than 2^31
+// points, so bit positions are 32-bit.  (Rows are at most 8192 points, 256
+// words, long.)
+__device__ __forceinline__ void list_words(const Grid& g, const uint32_t* __restrict__ bits,
+                                           unsigned lo, unsigned hi, int id0, unsigned short* list,
+                                           int* count) {
+  const int lane = threadIdx.x & 31;
+  const unsigned r0 = div_by(lo, g.mwr), rows = div_by(hi - 1u, g.mwr) - r0 + 1u;
+  const unsigned wr = (unsigned)g.wr;
+  const int n = (int)(hi - lo);
+  // the fewest rows a lane with which the block covers the range at once
+  const unsigned fit = (unsigned)kCountThreads / wr;
+  const unsigned depth = (rows + fit - 1u) / fit;
+  const unsigned items = (rows + depth - 1u) / depth * wr;
+  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, dz = nx * ny, P = (unsigned)g.P;
+  for (unsigned q0 = threadIdx.x & ~31u; q0 < items; q0 += kCountThreads) {
+    const bool mine = q0 + lane < items;
+    const unsigned q = mine ? q0 + lane : items - 1u;
+    const unsigned chunk = div_by(q, g.mwr), m = q - chunk * wr;
+    const unsigned r = r0 + chunk * depth;
+    const unsigned pmask = mine ? low_mask((int)nx - 32 * (int)m) : 0u;
+    unsigned j = r - div_by(r, g.mny) * ny;
+    unsigned w = r * wr + m - lo;  // the word's place in the range; before it: above n
+    unsigned pos = r * nx + 32u * m;
+    // any / all of the corner words of the row at bit `at`, both planes (the
+    // last plane: one); rows past the grid's end repeat its last words
+    auto row = [&](unsigned at, unsigned& any1, unsigned& all1) {
+      const unsigned p0 = at < P ? at : P - 1u;
+      const unsigned pz = p0 + dz < P ? p0 + dz : p0;
+      const uint32_t* const s0 = bits + (p0 >> 5);
+      const uint32_t* const sz = bits + (pz >> 5);
+      const uint32_t x0 = __ldg(s0), x1 = __ldg(s0 + 1), z0 = __ldg(sz), z1 = __ldg(sz + 1);
+      const uint32_t a = __funnelshift_r(x0, x1, p0), a1 = __funnelshift_rc(x0, x1, (p0 & 31u) + 1u);
+      const uint32_t c = __funnelshift_r(z0, z1, pz), c1 = __funnelshift_rc(z0, z1, (pz & 31u) + 1u);
+      any1 = a | a1 | c | c1;
+      all1 = a & a1 & c & c1;
+    };
+    unsigned any1, all1;
+    row(pos, any1, all1);
+#pragma unroll 4
+    for (unsigned d = 0; d < depth; ++d) {
+      const bool hy = j + 1u < ny;
+      unsigned any2, all2;
+      pos += nx;
+      row(pos, any2, all2);
+      const unsigned x = hy ? any1 | any2 : any1, y = hy ? all1 & all2 : all1;
+      push_word((x & ~y & pmask) != 0 && w < (unsigned)n, id0 + (int)w, list, count, lane);
+      any1 = any2;
+      all1 = all2;
+      j = hy ? j + 1u : 0u;
+      w += wr;
+    }
+  }
+}
+
+// K2a: one block per tile of kScanTile row words (grid-stride over tiles), in
+// two steps.  First every word's corner bits are compared: most words lie
+// wholly inside or outside, and the others are listed in shared memory.  Then
+// lane = listed word: its counts by word_tris.  (Counting in the first step
+// held every warp for its few words with a surface: 32 us for the 4.2 M words
+// of 512^3, now 25; a tile of the 201^3 Mandelbulb, nearly all of whose words
+// have one, 133 us, now 15.)  The block writes the tile's counts with
+// whole-line stores and its totals (triangles, crossing edges, active words)
+// to tile_tot[0 / 1 / 2][tile] for the scan.
+//
+// A set's tile with up to kCountSegments grids takes them one after another;
+// with more, each lane takes a word from its own grid: short ranges would
+// leave most of the block idle at each.
+template <bool SET>
+__global__ void __launch_bounds__(kCountThreads, 2) k_mc_count(GridSet S,
+                                                               const uint32_t* __restrict__ bits,
+                                                               uint32_t* __restrict__ wc,
+                                                               uint32_t* __restrict__ tile_tot,
+                                                               int tiles, int tile_begin,
+                                                               int tile_end) {
+  constexpr int kWarps = kCountThreads / 32;
+  __shared__ __align__(16) uint32_t s_wc[kScanTile];
+  __shared__ unsigned short s_list[kScanTile];
   __shared__ unsigned char s_nf[256];  // NumFaces, indexed by divergent case ids
-  __shared__ uint32_t s_red[24];
-  __shared__ long long s_keys[kStagedSlots];
-  s_nf[threadIdx.x] = (unsigned char)mc_num_tris(threadIdx.x);
-  const long long* keys =
-      stage_slot_keys(S, s_keys, [](const GridSlot& sl) { return sl.rw0; }) ? s_keys : nullptr;
+  __shared__ uint32_t s_sum[3];  // the tile's triangles, crossing edges and active words
+  __shared__ int s_count;
+  __shared__ long long s_keys[SET ? kStagedSlots : 1];
+  if (threadIdx.x < 256) s_nf[threadIdx.x] = (unsigned char)mc_num_tris(threadIdx.x);
+  const long long* keys = nullptr;
+  if (SET && stage_slot_keys(S, s_keys, [](const GridSlot& sl) { return sl.rw0; })) keys = s_keys;
   pdl_trigger();
   pdl_wait();  // the classification's bits
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int tile = tile_begin + blockIdx.x; tile < tile_end; tile += gridDim.x) {
-    uint32_t st = 0, sv = 0, sa = 0;
+    const long long t0 = (long long)tile * kScanTile;
+    const int words = (int)(t0 + kScanTile < S.rowwords ? kScanTile : S.rowwords - t0);
+    for (int i = threadIdx.x; i < kScanTile / 4; i += kCountThreads)
+      reinterpret_cast<uint4*>(s_wc)[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) s_count = 0;
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    // ---- step 1: the words with a crossing edge or an active cell ----------
+    if (!SET) {
+      list_words(S.one.g, bits, (unsigned)t0, (unsigned)t0 + (unsigned)words, 0, s_list, &s_count);
+    } else {
+      const long long te = t0 + words;
+      const int first = keys ? slot_search(keys, S.count, t0) : slot_of_rowword(S, t0);
+      const int past = first + kCountSegments;
+      if (past >= S.count || (keys ? keys[past] : __ldg(&S.slots[past].rw0)) >= te) {
+        for (int si = first; si < S.count; ++si) {
+          const GridSlot& sl = S.slots[si];
+          if (sl.rw0 >= te) break;
+          const Grid& g = sl.g;
+          const long long W = g.R * g.wr;
+          const long long lo = t0 > sl.rw0 ? t0 - sl.rw0 : 0, hi = te - sl.rw0 < W ? te - sl.rw0 : W;
+          if (lo < hi && g.nx >= 2 && g.ny >= 2 && g.nz >= 2)
+            list_words(g, bits + sl.word0, (unsigned)lo, (unsigned)hi, (int)(sl.rw0 + lo - t0),
+                       s_list, &s_count);
+        }
+      } else {
+        // many small grids: a word per lane, each from its own grid
 #pragma unroll 1
-    for (int e = 0; e < kScanItems / kCountWords; ++e) {
-      const long long g0 = (long long)tile * kScanTile + (long long)(threadIdx.x + 256 * e) * kCountWords;
-      // the slot of the warp's first group, searched once (the warp's
-      // groups are consecutive); every lane steps forward from it
-      const long long gw0 = g0 - (long long)(threadIdx.x & 31) * kCountWords;
-      const int s0 = S.count == 1 || gw0 >= S.rowwords
-                         ? 0
-                         : (keys ? slot_search(keys, S.count, gw0) : slot_of_rowword(S, gw0));
-      if (g0 >= S.rowwords) break;
-      int si, m;
-      unsigned r;
-      locate_word(S, g0, si, r, m, keys, s0);
-      const GridSlot& sl = S.count == 1 ? S.one : S.slots[si];
-      const Grid& g = sl.g;
-      uint32_t out[kCountWords] = {0, 0, 0, 0};
-      const bool cells = g.nx >= 2 && g.ny >= 2 && g.nz >= 2;
-      if (cells && m + kCountWords <= g.wr && g0 + kCountWords <= S.rowwords &&
-          (S.count == 1 || g0 + kCountWords <= sl.rw0 + (long long)g.R * g.wr)) {
-        // fast path: the four words lie in one row
-        const uint32_t* gb = bits + sl.word0;
-        int j, k;
-  split_row(g, r, j, k);
-        const bool hy = j < g.ny - 1, hz = k < g.nz - 1;
-        const long long dy = g.nx, dz = (long long)g.nx * g.ny;
-        const long long pos = (long long)r * g.nx + 32ll * m;
-        uint32_t a[4], a1[4], b[4] = {0, 0, 0, 0}, b1[4] = {0, 0, 0, 0}, c[4] = {0, 0, 0, 0},
-                 c1[4] = {0, 0, 0, 0}, d[4] = {0, 0, 0, 0}, d1[4] = {0, 0, 0, 0};
-        row_windows4(gb, pos, a, a1);
-        if (hy) row_windows4(gb, pos + dy, b, b1);
-        if (hz) row_windows4(gb, pos + dz, c, c1);
-        if (hy && hz) row_windows4(gb, pos + dy + dz, d, d1);
-        // most groups lie wholly inside or outside: every corner window of
-        // every word equal means no crossing edge and no active cell
-        uint32_t diff = 0;
-#pragma unroll
-        for (int q = 0; q < kCountWords; ++q) {
-          diff |= a[q] ^ a1[q];
-          if (hy) diff |= (a[q] ^ b[q]) | (a[q] ^ b1[q]);
-          if (hz) diff |= (a[q] ^ c[q]) | (a[q] ^ c1[q]);
-          if (hy && hz) diff |= (a[q] ^ d[q]) | (a[q] ^ d1[q]);
-        }
-        if (diff) {
-#pragma unroll
-          for (int q = 0; q < kCountWords; ++q) {
-            const CornerWords w{a[q], a1[q], b[q], b1[q], c[q], c1[q], d[q], d1[q]};
-            out[q] = packed_counts(w, hy, hz, low_mask(g.nx - 32 * (m + q)),
-                                   low_mask(g.nx - 1 - 32 * (m + q)), s_nf);
+        for (int e = 0; e < kScanTile / kCountThreads; ++e) {
+          const int id0 = (kWarps * e + warp) * 32, id = id0 + lane;
+          if (id0 >= words) break;  // uniform across the warp
+          // the slot of the warp's first word, searched once; every lane
+          // steps forward from it
+          const int s0 = keys ? slot_search(keys, S.count, t0 + id0) : slot_of_rowword(S, t0 + id0);
+          bool on = false;
+          if (id < words) {
+            const GridSlot& sl = S.slots[slot_after(S, keys, s0, t0 + id)];
+            const Grid& g = sl.g;
+            on = g.nx >= 2 && g.ny >= 2 && g.nz >= 2 &&
+                 word_differs(g, bits + sl.word0, (unsigned)(t0 + id - sl.rw0));
           }
+          push_word(on, id, s_list, &s_count, lane);
         }
-      } else {
-        // words that straddle a row or grid end: one at a time
-#pragma unroll
-        for (int q = 0; q < kCountWords; ++q) {
-          const long long gw = g0 + q;
-          if (gw >= S.rowwords) break;
-          int sq, mq;
-          unsigned rq;
-          locate_word(S, gw, sq, rq, mq, keys, si);
-          const GridSlot& slq = S.count == 1 ? S.one : S.slots[sq];
-          if (slq.g.nx >= 2 && slq.g.ny >= 2 && slq.g.nz >= 2) {
-            const WordBits wb = load_word_bits(slq.g, bits + slq.word0, rq, mq);
-            out[q] = packed_counts(wb.w, wb.hy, wb.hz, wb.pmask, wb.xmask, s_nf);
-          }
-        }
-      }
-      if (g0 + kCountWords <= S.rowwords) {
-        *reinterpret_cast<uint4*>(wc + g0) = make_uint4(out[0], out[1], out[2], out[3]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < kCountWords; ++q)
-          if (g0 + q < S.rowwords) wc[g0 + q] = out[q];
-      }
-#pragma unroll
-      for (int q = 0; q < kCountWords; ++q) {
-        st += out[q] >> 16;
-        sv += out[q] & 0xffffu;
-        sa += out[q] ? 1u : 0u;
       }
     }
-    block_sum3(st, sv, sa, s_red);
-    if (threadIdx.x == 0) {
-      tile_tot[tile] = st;
-      tile_tot[tiles + tile] = sv;
-      tile_tot[2 * tiles + tile] = sa;
+    __syncthreads();
+    // ---- step 2: lane = listed word ----------------------------------------
+    const int listed = s_count;
+#pragma unroll 1
+    for (int i0 = threadIdx.x & ~31; i0 < listed; i0 += kCountThreads) {
+      uint32_t out = 0;
+      if (i0 + lane < listed) {
+        const int id = s_list[i0 + lane];
+        int si, m;
+        unsigned r;
+        locate_word(S, t0 + id, si, r, m, keys);
+        const GridSlot& sl = SET ? S.slots[si] : S.one;
+        const WordBits wb = load_word_bits(sl.g, bits + sl.word0, r, m);
+        out = packed_counts(wb.w, wb.hy, wb.hz, wb.pmask, wb.xmask, s_nf);
+        s_wc[id] = out;
+      }
+      const uint32_t st = __reduce_add_sync(kFull, out >> 16), sv = __reduce_add_sync(kFull, out & 0xffffu);
+      const uint32_t sa = __popc(__ballot_sync(kFull, out != 0));
+      if (lane == 0) {
+        atomicAdd(&s_sum[0], st);
+        atomicAdd(&s_sum[1], sv);
+        atomicAdd(&s_sum[2], sa);
+      }
     }
+    __syncthreads();
+    if (words == kScanTile) {
+      for (int i = threadIdx.x; i < kScanTile / 4; i += kCountThreads)
+        reinterpret_cast<uint4*>(wc + t0)[i] = reinterpret_cast<const uint4*>(s_wc)[i];
+    } else {
+      for (int i = threadIdx.x; i < words; i += kCountThreads) wc[t0 + i] = s_wc[i];
+    }
+    if (threadIdx.x < 3) tile_tot[threadIdx.x * tiles + tile] = s_sum[threadIdx.x];
+    __syncthreads();  // s_wc, s_sum and the list are free
   }
 }
 
@@ -359,8 +452,7 @@ __global__ void __launch_bounds__(256) k_word_scan(long long rowwords,
       slab_act[B.n] = (uint32_t)(ea + ta);
     } else {
       info->error = ((T > 2147483647ll || V > 2147483647ll) ? kErrOverflow : 0) |
-                    ((abort && *(volatile const uint32_t*)abort) ? kErrTimeout : 0) |
-                    (*(volatile int*)&info->aborted ? kErrTimeout : 0);
+                    ((abort && *(volatile const uint32_t*)abort) ? kErrTimeout : 0);
       info->ticket = 0;
       info->done = 0;
     }
@@ -379,163 +471,16 @@ void launch_word_scan(long long rowwords, const uint32_t* wc, const uint32_t* ti
              act, info, 0, SlabBounds{}, (uint32_t*)nullptr, abort);
 }
 
-// K2a for grid sets: the same counts, with the triangles of the active
-// cells dealt across the warp.  Batches of small grids have short rows (the
-// 4-word groups straddle rows) and, with noisy fields, many active cells,
-// so a lane looping over its own words' active cells would hold its warp
-// for the busiest lane.  Here a lane gathers its 4 words' corner bits and
-// counts their crossing edges; the warp then deals the active cells of its
-// 128 words to the lanes, a cell per lane per round: each reads its word's
-// corner bits from the warp's staging area and adds NumFaces of its case to
-// the word's total there.  (For one large grid the per-lane loop is faster:
-// its surface is sparse, and this kernel's staging costs occupancy.)
-__global__ void __launch_bounds__(256) k_mc_count_dealt(GridSet S, const uint32_t* __restrict__ bits,
-                                                        uint32_t* __restrict__ wc,
-                                                        uint32_t* __restrict__ tile_tot, int tiles) {
-  constexpr int kSlots = 32 * kCountWords;  // words per warp step
-  __shared__ unsigned char s_nf[256];        // NumFaces
-  __shared__ uint32_t s_red[24];
-  __shared__ long long s_keys[kStagedSlots];
-  __shared__ uint32_t s_win[8][8 * kSlots];  // corner word f of slot (4 lane + q) at f * kSlots + slot
-  __shared__ uint32_t s_tri[8][kSlots];      // triangles of slot
-  s_nf[threadIdx.x] = (unsigned char)mc_num_tris(threadIdx.x);
-  const long long* keys =
-      stage_slot_keys(S, s_keys, [](const GridSlot& sl) { return sl.rw0; }) ? s_keys : nullptr;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  uint32_t* const win = s_win[wib];
-  uint32_t* const tri = s_tri[wib];
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    uint32_t st = 0, sv = 0, sa = 0;
-#pragma unroll 1
-    for (int e = 0; e < kScanItems / kCountWords; ++e) {
-      const long long gw0 = (long long)tile * kScanTile + (long long)(256 * e + 32 * wib) * kCountWords;
-      if (gw0 >= S.rowwords) break;  // uniform across the warp
-      const long long g0 = gw0 + (long long)lane * kCountWords;
-      const int s0 = keys ? slot_search(keys, S.count, gw0) : slot_of_rowword(S, gw0);
-      // ---- lane = 4 words: corner bits, crossing edges, active cells ------
-      CornerWords w[kCountWords];
-      uint32_t v[kCountWords], am[kCountWords], t[kCountWords] = {0, 0, 0, 0};
-#pragma unroll
-      for (int q = 0; q < kCountWords; ++q) {
-        w[q] = CornerWords{};
-        v[q] = am[q] = 0u;
-        const long long gw = g0 + q;
-        if (gw < S.rowwords) {
-          int sq, mq;
-          unsigned rq;
-          locate_word(S, gw, sq, rq, mq, keys, s0);
-          const GridSlot& slq = S.slots[sq];
-          if (slq.g.nx >= 2 && slq.g.ny >= 2 && slq.g.nz >= 2) {
-            const WordBits wb = load_word_bits(slq.g, bits + slq.word0, rq, mq);
-            w[q] = wb.w;
-            int vv = __popc((wb.w.a ^ wb.w.a1) & wb.xmask);
-            if (wb.hy) vv += __popc((wb.w.a ^ wb.w.b) & wb.pmask);
-            if (wb.hz) vv += __popc((wb.w.a ^ wb.w.c) & wb.pmask);
-            v[q] = (uint32_t)vv;
-            am[q] = (wb.hy && wb.hz) ? active_cells(wb.w, wb.xmask) : 0u;
-          }
-        }
-      }
-      // ---- lane = active cell -------------------------------------------
-      const int cnt = __popc(am[0]) + __popc(am[1]) + __popc(am[2]) + __popc(am[3]);
-      int pre = cnt;  // inclusive scan of the lanes' active cells
-#pragma unroll
-      for (int dd = 1; dd < 32; dd <<= 1) {
-        const int y = __shfl_up_sync(kFull, pre, dd);
-        if (lane >= dd) pre += y;
-      }
-      const int total = __shfl_sync(kFull, pre, 31);
-      pre -= cnt;
-      if (total > 0) {
-#pragma unroll
-        for (int q = 0; q < kCountWords; ++q) {
-          const int slot = kCountWords * lane + q;
-          tri[slot] = 0u;
-          if (am[q]) {
-            win[0 * kSlots + slot] = w[q].a;
-            win[1 * kSlots + slot] = w[q].a1;
-            win[2 * kSlots + slot] = w[q].b;
-            win[3 * kSlots + slot] = w[q].b1;
-            win[4 * kSlots + slot] = w[q].c;
-            win[5 * kSlots + slot] = w[q].c1;
-            win[6 * kSlots + slot] = w[q].d;
-            win[7 * kSlots + slot] = w[q].d1;
-          }
-        }
-        __syncwarp();
-        for (int t0 = 0; t0 < total; t0 += 32) {
-          const int tt = t0 + lane;
-          int s = 0;  // the lane holding cell tt: the last s with pre[s] <= tt
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1) {
-            const int ps = __shfl_sync(kFull, pre, s + step);
-            if (ps <= tt) s += step;
-          }
-          int rnk = tt - __shfl_sync(kFull, pre, s);
-          const uint32_t m0 = __shfl_sync(kFull, am[0], s), m1 = __shfl_sync(kFull, am[1], s),
-                         m2 = __shfl_sync(kFull, am[2], s), m3 = __shfl_sync(kFull, am[3], s);
-          if (tt < total) {
-            // the word q of lane s holding the cell, and the cell's rank in it
-            int q = 0;
-            uint32_t mq = m0;
-            const int c0 = __popc(m0), c01 = c0 + __popc(m1), c012 = c01 + __popc(m2);
-            if (rnk >= c012) {
-              q = 3;
-              mq = m3;
-              rnk -= c012;
-            } else if (rnk >= c01) {
-              q = 2;
-              mq = m2;
-              rnk -= c01;
-            } else if (rnk >= c0) {
-              q = 1;
-              mq = m1;
-              rnk -= c0;
-            }
-            const int slot = kCountWords * s + q;
-            const CornerWords cw{win[0 * kSlots + slot], win[1 * kSlots + slot],
-                                 win[2 * kSlots + slot], win[3 * kSlots + slot],
-                                 win[4 * kSlots + slot], win[5 * kSlots + slot],
-                                 win[6 * kSlots + slot], win[7 * kSlots + slot]};
-            atomicAdd(&tri[slot], (uint32_t)s_nf[case_of(cw, nth_bit(mq, rnk))]);
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kCountWords; ++q) t[q] = tri[kCountWords * lane + q];
-        __syncwarp();
-      }
-#pragma unroll
-      for (int q = 0; q < kCountWords; ++q) {
-        const uint32_t out = (t[q] << 16) | v[q];
-        if (g0 + q < S.rowwords) wc[g0 + q] = out;
-        st += t[q];
-        sv += v[q];
-        sa += out ? 1u : 0u;
-      }
-    }
-    block_sum3(st, sv, sa, s_red);
-    if (threadIdx.x == 0) {
-      tile_tot[tile] = st;
-      tile_tot[tiles + tile] = sv;
-      tile_tot[2 * tiles + tile] = sa;
-    }
-  }
-}
-
 void launch_mc_scan(const GridSet& S, const uint32_t* bits, const WordOffsets& o, Info* info,
-                    int num_sms, cudaStream_t s, int dealt) {
+                    int num_sms, cudaStream_t s) {
   const int tiles = word_scan_tiles(S.rowwords);
-  // the dealt pass reads the device slot table, which only grid sets have
-  if (S.count == 1 && launch_mc_count_staged(S.one.g, bits, bit_words(S.one.g.P), o, info, num_sms, s)) {
-    // one grid: each tile's bits staged in shared memory
-  } else if (S.count > 1 && dealt != 0) {
-    const int b1 = resident_blocks(k_mc_count_dealt, 256, 0, num_sms, tiles, kPassCount);
-    k_mc_count_dealt<<<b1, 256, 0, s>>>(S, bits, o.wc, o.tile, tiles);
-  } else {
-    const int b1 = resident_blocks(k_mc_count, 256, 0, num_sms, tiles, kPassCount);
-    k_mc_count<<<b1, 256, 0, s>>>(S, bits, o.wc, o.tile, tiles, 0, tiles);
-  }
+  const auto kernel = S.count > 1 ? k_mc_count<true> : k_mc_count<false>;
+  // a block a tile, unless other frames are to find room on the SMs
+  const int b1 = tuned_blocks_per_sm(kPassCount) > 0
+                     ? resident_blocks(kernel, kCountThreads, 0, num_sms, tiles, kPassCount)
+                     : tiles;
+  launch_pdl(kernel, (unsigned)b1, (unsigned)kCountThreads, 0, s, S, bits, o.wc, o.tile, tiles, 0,
+             tiles);
   launch_word_scan(S.rowwords, o.wc, o.tile, o.wt, o.wv, o.act, info, s);
 }
 
@@ -546,8 +491,8 @@ void launch_mc_scan_slab(const GridSet& S, const uint32_t* bits, const WordOffse
                          int pass, int num_sms, cudaStream_t s, cudaEvent_t after_count) {
   const int tiles = word_scan_tiles(S.rowwords);
   const int n = tile_end - tile_begin;
-  const int b1 = resident_blocks(k_mc_count, 256, 0, num_sms, n, pass);
-  k_mc_count<<<b1, 256, 0, s>>>(S, bits, o.wc, o.tile, tiles, tile_begin, tile_end);
+  const int b1 = resident_blocks(k_mc_count<false>, kCountThreads, 0, num_sms, n, pass);
+  k_mc_count<false><<<b1, kCountThreads, 0, s>>>(S, bits, o.wc, o.tile, tiles, tile_begin, tile_end);
   if (after_count) cudaEventRecord(after_count, s);
   k_word_scan<true><<<n, 256, 0, s>>>(S.rowwords, o.wc, o.tile, tiles, o.wt, o.wv, o.act, info,
                                       tile_begin, B, slab_act, nullptr);

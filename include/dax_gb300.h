@@ -44,8 +44,7 @@ typedef enum dax_gb300_status {
   /* an output buffer is smaller than the result; nothing was written */
   DAX_GB300_ERROR_CAPACITY = 5,
   /* a bounded device-side wait gave up (the fused count pass's blocks wait
-     on one another; the staged count waits for its bulk copies); the count
-     pass has no result and the generate pass writes nothing.  The single-pass
+     on one another); the count pass has no result and the generate pass writes nothing.  The single-pass
      integer scan, StreamCompact and Unique (whose tiles wait on the sums of
      earlier tiles) report it when their total or count is read */
   DAX_GB300_ERROR_TIMEOUT = 6,
@@ -173,7 +172,7 @@ int dax_gb300_mc_classify_count(const dax_gb300_uniform_grid* grid, const float*
 size_t dax_gb300_mc_scratch_bytes(const dax_gb300_uniform_grid* grid);
 
 /* Classify every point, count triangles and crossing edges per row word and
- * scan them (a classification, a staged count and a reduce-then-scan
+ * scan them (a classification, a count and a reduce-then-scan
  * launch; or the fused count, dax_gb300_set_fused_count): everything
  * DispatcherGenerateInterpolatedCells::GenerateNewTopology does before its
  * generate worklet (dax/cont/DispatcherGenerateInterpolatedCells.h:178-223).
@@ -526,7 +525,8 @@ int dax_gb300_mc_batch_field_adjoint(const dax_gb300_mc_batch* batch, const void
                                      void* stream);
 
 /* Sets (emit_batch 1..32, 0 = default 16; dealt_count 1, 0, -1 = default)
- * or reads a plan's configuration. */
+ * or reads a plan's configuration.  dealt_count is kept and read back; grid
+ * sets have one count pass, so it selects nothing. */
 int dax_gb300_mc_batch_set_config(dax_gb300_mc_batch* batch, int emit_batch, int dealt_count);
 int dax_gb300_mc_batch_get_config(const dax_gb300_mc_batch* batch, int* emit_batch,
                                   int* dealt_count);
