@@ -28,38 +28,74 @@ __device__ __forceinline__ float magsq3(float x, float y, float z) {
 
 // worklet::Mandlebulb (Benchmarks/Mandlebulb/Worklets.h:65-109): the escape
 // iteration of pos -> pos^10 + c (White and Nylander's power, :92-108), 0
-// when c itself is outside radius sqrt(2), at most 35.
-__device__ float mandelbulb_value(float cx, float cy, float cz) {
-  float x = cx, y = cy, z = cz;
-  if (magsq3(x, y, z) > 2.0f) return 0.0f;
-  for (int i = 1; i < 35; ++i) {
-    const float r2 = magsq3(x, y, z);
-    const float t = __fsqrt_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)));
-    const float thetaN = __fmul_rn(10.0f, atan2f(t, z));
-    const float phiN = __fmul_rn(10.0f, atan2f(y, z));
-    const float powR = powf(r2, 5.0f);
-    float st, ct;  // sincosf: bit for bit sinf and cosf (checked over every float on GB300)
-    sincosf(thetaN, &st, &ct);
-    const float px = __fmul_rn(powR, __fmul_rn(st, tanf(phiN)));
-    const float py = __fmul_rn(powR, __fmul_rn(st, sinf(phiN)));
-    const float pz = __fmul_rn(powR, ct);
-    x = __fadd_rn(px, cx);
-    y = __fadd_rn(py, cy);
-    z = __fadd_rn(pz, cz);
-    if (magsq3(x, y, z) > 2.0f) return (float)i;
-  }
-  return 35.0f;
+// when c itself is outside radius sqrt(2), at most 35.  One step of it.
+__device__ __forceinline__ void mandelbulb_step(float& x, float& y, float& z, float cx, float cy,
+                                                float cz) {
+  const float r2 = magsq3(x, y, z);
+  const float t = __fsqrt_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)));
+  const float thetaN = __fmul_rn(10.0f, atan2f(t, z));
+  const float phiN = __fmul_rn(10.0f, atan2f(y, z));
+  const float powR = powf(r2, 5.0f);
+  float st, ct;  // sincosf: bit for bit sinf and cosf (checked over every float on GB300)
+  sincosf(thetaN, &st, &ct);
+  const float px = __fmul_rn(powR, __fmul_rn(st, tanf(phiN)));
+  const float py = __fmul_rn(powR, __fmul_rn(st, sinf(phiN)));
+  const float pz = __fmul_rn(powR, ct);
+  x = __fadd_rn(px, cx);
+  y = __fadd_rn(py, cy);
+  z = __fadd_rn(pz, cz);
 }
 
+// Bound by arithmetic: two arctangents, a power, a sine and cosine, a tangent
+// and a sine a step, 1 to 34 steps a point.  With a point per lane a warp
+// steps until its slowest lane is done, so a lane that is done takes the
+// block's next point instead (its tiles of 256 points, strided by the grid,
+// in order, from a counter in shared memory), once kRefill lanes wait.
+constexpr int kRefill = 4;
+
 __global__ void __launch_bounds__(256) k_mandelbulb_field(Grid g, float* __restrict__ out) {
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < g.P;
-       p += (long long)gridDim.x * blockDim.x) {
-    const unsigned row = (unsigned)(p / g.nx);
-    const int i = (int)(p - (long long)row * g.nx);
-    int j, k;
-    split_row(g, row, j, k);
-    out[p] = mandelbulb_value(coord(g.ox, g.sx, i, g.mx), coord(g.oy, g.sy, j, g.my),
-                              coord(g.oz, g.sz, k, g.mz));
+  __shared__ unsigned s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const unsigned P = (unsigned)g.P, tiles = (P + 255u) / 256u;
+  const unsigned mine = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 256u;  // points, past P too
+  float x = 0, y = 0, z = 0, cx = 0, cy = 0, cz = 0;
+  unsigned p = 0;
+  int i = 0;  // the step the lane is at; 0: it has no point
+  bool more = true;
+  while (true) {
+    const unsigned idle = __ballot_sync(kFull, i == 0);
+    if (more && __popc(idle) >= kRefill) {
+      unsigned n = 0;
+      if (lane == 0) n = atomicAdd(&s_next, (unsigned)__popc(idle));
+      n = __shfl_sync(kFull, n, 0);
+      more = n + (unsigned)__popc(idle) < mine;
+      n += (unsigned)__popc(idle & ((1u << lane) - 1u));
+      p = i == 0 ? ((n >> 8) * gridDim.x + blockIdx.x) * 256u + (n & 255u) : p;
+      if (i == 0 && n < mine && p < P) {
+        const unsigned row = p / (unsigned)g.nx;
+        int j, k;
+        split_row(g, row, j, k);
+        x = cx = coord(g.ox, g.sx, (int)(p - row * (unsigned)g.nx), g.mx);
+        y = cy = coord(g.oy, g.sy, j, g.my);
+        z = cz = coord(g.oz, g.sz, k, g.mz);
+        if (magsq3(x, y, z) > 2.0f) out[p] = 0.0f;
+        else i = 1;
+      }
+    } else if (idle == kFull) {
+      break;
+    }
+    if (i > 0) {
+      mandelbulb_step(x, y, z, cx, cy, cz);
+      const bool escaped = magsq3(x, y, z) > 2.0f;
+      if (escaped || i == 34) {
+        out[p] = escaped ? (float)i : 35.0f;
+        i = 0;
+      } else {
+        ++i;
+      }
+    }
   }
 }
 
