@@ -1,6 +1,7 @@
 // The Mandelbulb benchmark's compute pipeline (Benchmarks/Mandlebulb): the
-// escape-iteration point field, the clip-and-count worklet of its cut view,
-// and the per-point normals and colours of the extracted surface.  The
+// escape-iteration point field and the per-point normals and colours of the
+// extracted surface (the clip-and-count worklet of its cut view is the third
+// mode of k_cell_count, classify.cu).  The
 // surface itself is the marching-cubes pipeline (extractSurface,
 // Mandlebulb.cxx:105-118) or the count-array-driven generate of the cut
 // (extractCut, Mandlebulb.cxx:126-157); its GLUT/shader display is replaced
@@ -16,7 +17,6 @@
 #include "common.cuh"
 #include "coolwarm_table.h"
 #include "kernels.cuh"
-#include "mc_case.cuh"
 
 namespace daxgb {
 
@@ -140,39 +140,6 @@ __global__ void __launch_bounds__(256) k_colors_and_norms(const float* __restric
   }
 }
 
-// worklet::MandlebulbClipCount (Worklets.h:112-170): a cell's marching-cubes
-// triangle count when one of its points lies beyond the plane,
-// dot(N, p - O) > dot(N, L); otherwise 0.  One thread per cell.
-__global__ void __launch_bounds__(256) k_mandelbulb_clip_count(Grid g, const float* __restrict__ f,
-                                                               float iso, float3 o, float3 n,
-                                                               float loc, unsigned long long mcx,
-                                                               unsigned long long mcy,
-                                                               long long C,
-                                                               int32_t* __restrict__ count) {
-  __shared__ unsigned char s_nf[256];
-  s_nf[threadIdx.x] = (unsigned char)mc_num_tris(threadIdx.x);
-  __syncthreads();
-  const unsigned cx = (unsigned)(g.nx - 1), cy = (unsigned)(g.ny - 1);
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < C;
-       c += (long long)gridDim.x * blockDim.x) {
-    const unsigned r = div_by((unsigned)c, mcx);
-    const int i = (int)((unsigned)c - r * cx);
-    const unsigned kk = div_by(r, mcy);
-    const int k = (int)kk, j = (int)(r - kk * cy);
-    const long long p0 = ((long long)k * g.ny + j) * g.nx + i;
-    const long long sy = g.nx, sz = (long long)g.nx * g.ny;
-    bool in = false;
-    int cs = 0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int dx = (0x66 >> q) & 1, dy = (0xCC >> q) & 1, dz = q >> 2;
-      in = in || plane_value(g, o, n, i + dx, j + dy, k + dz) > loc;
-      cs |= (__ldg(f + p0 + dx + dy * sy + dz * sz) > iso ? 1 : 0) << q;
-    }
-    count[c] = in ? (int32_t)s_nf[cs] : 0;
-  }
-}
-
 void launch_mandelbulb_field(const Grid& g, float* out, int num_sms, cudaStream_t s) {
   const int b = resident_blocks(k_mandelbulb_field, 256, 0, num_sms, (g.P + 255) / 256);
   k_mandelbulb_field<<<b, 256, 0, s>>>(g, out);
@@ -182,15 +149,6 @@ void launch_colors_and_norms(const float* verts, long long nv, float* norms, uin
                              int num_sms, cudaStream_t s) {
   const int b = resident_blocks(k_colors_and_norms, 256, 0, num_sms, (nv + 255) / 256);
   k_colors_and_norms<<<b, 256, 0, s>>>(verts, nv, norms, colors);
-}
-
-void launch_mandelbulb_clip_count(const Grid& g, const float* f, float iso, float3 o, float3 n,
-                                  float loc, int32_t* count, int num_sms, cudaStream_t s) {
-  const long long C = (long long)(g.nx - 1) * (g.ny - 1) * (g.nz - 1);
-  const int b = resident_blocks(k_mandelbulb_clip_count, 256, 0, num_sms, (C + 255) / 256);
-  k_mandelbulb_clip_count<<<b, 256, 0, s>>>(g, f, iso, o, n, loc,
-                                            div_multiplier((unsigned)(g.nx - 1)),
-                                            div_multiplier((unsigned)(g.ny - 1)), C, count);
 }
 
 }  // namespace daxgb

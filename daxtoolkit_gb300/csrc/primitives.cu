@@ -282,8 +282,8 @@ void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, voi
 // 32-bit sums, two such words (low and high halves) for 64-bit sums.
 constexpr unsigned kStAgg = 1u, kStInc = 2u;
 constexpr size_t kScanHead = 64;
-constexpr int kSThreads = 256;                                // compute threads
-constexpr int kSChunks = 16;                                  // 16-byte chunks a thread
+constexpr int kSThreads = 512;                                // compute threads
+constexpr int kSChunks = 8;                                   // 16-byte chunks a thread
 constexpr unsigned kSTileBytes = 16u * kSChunks * kSThreads;  // 64 KB
 constexpr int kSStages = 3;
 
