@@ -8,7 +8,7 @@
 //               s_a * 0.25 * dL/dg_c[a] / width_c[a]
 // with s_a = +1 when p is on the cell's upper face along a, else -1.
 // k_grad_adjoint marches along z over a warp tile (31 point columns x kAdjBand
-// point rows x kSeg planes).  Per cell plane and cell row jc it forms, at
+// point rows x a segment of planes).  Per cell plane and cell row jc it forms, at
 // point column i, the x-pair sums
 //     Hx = ax(i-1) - ax(i),   Hy = ay(i-1) + ay(i),   Hz = az(i-1) + az(i)
 // (a = 0.25 dL/dg / width, zero outside the cells), so that a point row j
@@ -51,101 +51,182 @@ __device__ __forceinline__ float width_z(const Grid& g, int k) {
 // Lane L of a warp tile holds cell column ic = 31 xw - 1 + L and outputs
 // point column ic + 1 (lanes 0..30), whose -x cell is its own column and
 // whose +x cell is lane L + 1's.  Per cell plane the tile's kAdjBand + 1 cell
-// rows (jc = j0 - 1 + t) are loaded together (three 4-byte loads per cell,
-// 384 contiguous bytes per warp load), then reduced row by row into the
-// point rows t = 0..kAdjBand-1 they bracket.
-__device__ __forceinline__ void grad_adjoint_task(const Grid& g, const float* __restrict__ dg,
-                                                  float* __restrict__ out, const MarchTiles& mt,
-                                                  long long task) {
+// rows (jc = j0 - 1 + t), 96 consecutive floats each, are copied into the
+// warp's ring in shared memory (one 16-byte cp.async a lane and row, from the
+// 16-byte boundary at or before the row's first float; rows outside the grid
+// zero-filled) while the plane before is reduced row by row into the point
+// rows t = 0..kAdjBand-1 it brackets.
+//
+// Bound by HBM.  Three strided loads a cell held in registers, no plane ahead,
+// in segments of 32 planes took 135 us for 385 x 321 x 289 (567 MB, 85 us at
+// the copy bandwidth), now 121, and 109 from a clean L2.  (4-byte copies, 73
+// instructions a row against 42, measured no faster than the loads.)
+//
+// A block is one warp: the tile's place is then uniform over the block, and
+// the row addresses and tests are scalar work.
+constexpr int kAdjRows = kAdjBand + 1;
+constexpr int kAdjPitch = 100;                  // floats of a row in the ring: 96 and up to 3 before
+constexpr int kAdjSlot = kAdjRows * kAdjPitch;  // of a plane
+constexpr size_t kAdjSmem = 2 * kAdjSlot * sizeof(float);
+
+// EDGE: the tile has cell columns outside the grid (their floats in the ring
+// belong to other rows), or the last point plane, which no cells lie above.
+template <bool EDGE>
+__device__ __forceinline__ void grad_adjoint_tile(const Grid& g, const float* __restrict__ dg,
+                                                  float* __restrict__ out, int xw, int j0, int k0,
+                                                  int k1) {
+  extern __shared__ __align__(16) float s_ring[];  // [2][kAdjSlot]
   const int lane = threadIdx.x & 31;
-  if (task >= mt.tasks) return;  // the whole warp leaves; no block barrier follows
-  const int xw = (int)(task % mt.nxw);
-  const long long t2 = task / mt.nxw;
-  const int band = (int)(t2 % mt.nband), seg = (int)(t2 / mt.nband);
+  float* const ring = s_ring;
   const int cx = g.nx - 1, cy = g.ny - 1, cz = g.nz - 1;
-  const int ic = kMarchCols * xw - 1 + lane;  // this lane's cell column
+  const int ic0 = kMarchCols * xw - 1, ic = ic0 + lane;  // this lane's cell column
   const bool col = ic >= 0 && ic < cx;
   const int i = ic + 1;                       // this lane's point column
   const bool pcol = lane < kMarchCols && i < g.nx;
-  const int j0 = band * kAdjBand;
-  const int k0 = seg * kSeg, k1 = min(k0 + kSeg, g.nz);
 
   // 0.25 / width of this lane's cell column and of the tile's cell rows
   const float rx = col ? __fdiv_rn(0.25f, width_x(g, ic)) : 0.0f;
-  float ry[kAdjBand + 1];
+  float ry[kAdjRows];
 #pragma unroll
-  for (int t = 0; t <= kAdjBand; ++t) {
+  for (int t = 0; t < kAdjRows; ++t) {
     const int jc = j0 - 1 + t;
     ry[t] = (jc >= 0 && jc < cy) ? __fdiv_rn(0.25f, width_y(g, jc)) : 0.0f;
   }
 
+  // float indices count from the 16-byte boundary at or before dg; `end` is
+  // past the grid's last gradient
+  const int off = (int)((reinterpret_cast<uintptr_t>(dg) >> 2) & 3);
+  const float* const base = dg - off;
+  const long long end = 3ll * cx * cy * cz + off;
+  const long long first0 = 3 * ((long long)ic0 + (long long)cx * (j0 - 1)) + off;
+  const long long plane = 3ll * cx * cy;
+  const unsigned ring_at = (unsigned)__cvta_generic_to_shared(ring) + 16u * (unsigned)lane;
+  // the rows of the tile inside the grid; the others hold zeros in both slots
+  const int t0 = j0 == 0 ? 1 : 0, t1 = min(kAdjRows, cy + 1 - j0);
+  const bool lane_on = lane < kAdjPitch / 4;
+  if (t0 > 0 || t1 < kAdjRows) {
+    for (int q = lane; q < 2 * kAdjSlot; q += 32) ring[q] = 0.0f;
+    __syncwarp();
+  }
+  const unsigned pitch = 3u * (unsigned)cx;  // rows are at most 8191 cells
+  auto issue = [&](int kc) {
+    const long long first = first0 + plane * kc, at = first & ~3ll;  // the plane's first row
+    const unsigned shift = (unsigned)first & 3u;
+    const float* const p = base + at + 4 * lane;
+    const unsigned slot = ring_at + (unsigned)(kc & 1) * (kAdjSlot * 4);
+    if (t0 == 0 && t1 == kAdjRows && at + (kAdjBand * pitch + kAdjPitch + 4) <= end) {
+#pragma unroll
+      for (int t = 0; t < kAdjRows; ++t)
+        if (lane_on)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(slot + kAdjPitch * 4 * t),
+                       "l"(p + ((shift + pitch * t) & ~3u))
+                       : "memory");
+    } else {
+      // rows that start before the array's first floats or end past its last
+      // ones are cut to what there is
+#pragma unroll 1
+      for (int t = t0; t < t1; ++t) {
+        const long long rel = (shift + pitch * t) & ~3u, q = at + rel + 4 * lane, left = end - q;
+        const int bytes = q >= 0 && left > 0 ? (left < 4 ? 4 * (int)left : 16) : 0;
+        if (lane_on)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(slot + kAdjPitch * 4 * t),
+                       "l"(bytes ? p + rel : base), "r"(bytes)
+                       : "memory");
+      }
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+
   float U[kAdjBand];  // (P + Z) of the previous cell plane, per point row
 #pragma unroll
   for (int t = 0; t < kAdjBand; ++t) U[t] = 0.0f;
-  for (int kc = k0 > 0 ? k0 - 1 : k0; kc < k1; ++kc) {
-    float gx[kAdjBand + 1], gy[kAdjBand + 1], gz[kAdjBand + 1];
-    float rz = 0.0f;
-    if (kc < cz) {
-      rz = __fdiv_rn(0.25f, width_z(g, kc));
-#pragma unroll
-      for (int t = 0; t <= kAdjBand; ++t) {
-        const int jc = j0 - 1 + t;
-        const bool ok = col && jc >= 0 && jc < cy;
-        const float* c = dg + 3 * ((long long)ic + (long long)cx * (jc + (long long)cy * kc));
-        gx[t] = ok ? __ldg(c) : 0.0f;
-        gy[t] = ok ? __ldg(c + 1) : 0.0f;
-        gz[t] = ok ? __ldg(c + 2) : 0.0f;
-      }
-    } else {
-#pragma unroll
-      for (int t = 0; t <= kAdjBand; ++t) gx[t] = gy[t] = gz[t] = 0.0f;
-    }
-    const bool emit = kc >= k0;
+  const int kb = k0 > 0 ? k0 - 1 : k0;
+  const int rows = pcol ? min(kAdjBand, g.ny - j0) : 0;  // this lane's outputs of a plane
+  float* o = out + ((long long)i + (long long)g.nx * (j0 + (long long)g.ny * kb));
+  const int nx = g.nx;
+  issue(kb);
+  commit();
+  for (int kc = kb; kc < k1; ++kc, o += (long long)g.nx * g.ny) {
+    if (kc + 1 < k1 && kc + 1 < cz) issue(kc + 1);
+    commit();
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncwarp();  // every lane's copies of plane kc have landed
+    const float* const slot = ring + (kc & 1) * kAdjSlot + 3 * lane;
+    const unsigned shift = (unsigned)(first0 + plane * kc) & 3u;
+    const bool cells = kc < cz;  // the last point plane has no cells above it
+    auto cell = [&](int t, float& gx, float& gy, float& gz) {
+      const float* const c = slot + (kAdjPitch * t + ((shift + pitch * t) & 3u));
+      gx = c[0];
+      gy = c[1];
+      gz = c[2];
+      if (EDGE && !(col && cells)) gx = gy = gz = 0.0f;
+    };
+    const float rz = EDGE && !cells ? 0.0f : __fdiv_rn(0.25f, width_z(g, kc));
+    const int nr = kc >= k0 ? rows : 0;
     // x-pair sums of cell row t at this lane's point column
     float hx0, hy0, hz0;
     {
-      const float ax = __fmul_rn(gx[0], rx);
+      float gx, gy, gz;
+      cell(0, gx, gy, gz);
+      const float ax = __fmul_rn(gx, rx);
       hx0 = __fsub_rn(ax, __shfl_down_sync(kFull, ax, 1));
-      hy0 = __fmul_rn(__fadd_rn(gy[0], __shfl_down_sync(kFull, gy[0], 1)), ry[0]);
-      hz0 = __fmul_rn(__fadd_rn(gz[0], __shfl_down_sync(kFull, gz[0], 1)), rz);
+      hy0 = __fmul_rn(__fadd_rn(gy, __shfl_down_sync(kFull, gy, 1)), ry[0]);
+      hz0 = __fmul_rn(__fadd_rn(gz, __shfl_down_sync(kFull, gz, 1)), rz);
     }
 #pragma unroll
     for (int t = 0; t < kAdjBand; ++t) {
-      const float ax = __fmul_rn(gx[t + 1], rx);
+      float gx, gy, gz;
+      cell(t + 1, gx, gy, gz);
+      const float ax = __fmul_rn(gx, rx);
       const float hx1 = __fsub_rn(ax, __shfl_down_sync(kFull, ax, 1));
-      const float hy1 =
-          __fmul_rn(__fadd_rn(gy[t + 1], __shfl_down_sync(kFull, gy[t + 1], 1)), ry[t + 1]);
-      const float hz1 = __fmul_rn(__fadd_rn(gz[t + 1], __shfl_down_sync(kFull, gz[t + 1], 1)), rz);
+      const float hy1 = __fmul_rn(__fadd_rn(gy, __shfl_down_sync(kFull, gy, 1)), ry[t + 1]);
+      const float hz1 = __fmul_rn(__fadd_rn(gz, __shfl_down_sync(kFull, gz, 1)), rz);
       const float P = __fadd_rn(__fadd_rn(hx0, hx1), __fsub_rn(hy0, hy1));
       const float Z = __fadd_rn(hz0, hz1);
-      const int j = j0 + t;
-      if (emit && pcol && j < g.ny)
-        out[(long long)i + (long long)g.nx * (j + (long long)g.ny * kc)] =
-            __fadd_rn(U[t], __fsub_rn(P, Z));
+      if (t < nr) o[t * nx] = __fadd_rn(U[t], __fsub_rn(P, Z));
       U[t] = __fadd_rn(P, Z);
       hx0 = hx1;
       hy0 = hy1;
       hz0 = hz1;
     }
+    __syncwarp();  // the slot is free for plane kc + 2
   }
 }
 
-__global__ void __launch_bounds__(kMarchWarps * 32, kAdjMinBlocks)
+__device__ __forceinline__ void grad_adjoint_task(const Grid& g, const float* __restrict__ dg,
+                                                  float* __restrict__ out, const MarchTiles& mt,
+                                                  long long task) {
+  if (task >= mt.tasks) return;  // the whole warp leaves; no block barrier follows
+  const int xw = (int)(task % mt.nxw);
+  const long long t2 = task / mt.nxw;
+  const int j0 = (int)(t2 % mt.nband) * kAdjBand, k0 = (int)(t2 / mt.nband) * mt.seg;
+  const int k1 = min(k0 + mt.seg, g.nz);
+  if (xw == 0 || kMarchCols * xw + 31 > g.nx - 1 || k1 == g.nz)
+    grad_adjoint_tile<true>(g, dg, out, xw, j0, k0, k1);
+  else
+    grad_adjoint_tile<false>(g, dg, out, xw, j0, k0, k1);
+}
+
+__host__ __device__ inline int adj_nxw(const Grid& g) { return (g.nx + kMarchCols - 1) / kMarchCols; }
+__host__ __device__ inline int adj_bands(const Grid& g) { return (g.ny + kAdjBand - 1) / kAdjBand; }
+__host__ __device__ inline MarchTiles adj_set_tiles(const Grid& g) {
+  return march_tiles(adj_nxw(g), adj_bands(g), g.nz, (g.nz + kSeg - 1) / kSeg);
+}
+
+__global__ void __launch_bounds__(32, kAdjMinBlocks)
     k_grad_adjoint(Grid g, const float* __restrict__ dg, float* __restrict__ out, MarchTiles mt) {
-  grad_adjoint_task(g, dg, out, mt, (long long)blockIdx.x * kMarchWarps + (threadIdx.x >> 5));
+  grad_adjoint_task(g, dg, out, mt, blockIdx.x);
 }
 
 // A grid set: the block's grid (block0 as in k_cell_gradient_set); cell
 // gradients and the output field are concatenated over the set.
-__global__ void __launch_bounds__(kMarchWarps * 32, kAdjMinBlocks)
+__global__ void __launch_bounds__(32, kAdjMinBlocks)
     k_grad_adjoint_set(GridSet S, const long long* __restrict__ block0,
                        const float* __restrict__ dg, float* __restrict__ out) {
   const int si = block_slot(block0, S.count, blockIdx.x);
   const Grid g = S.slots[si].g;
-  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0,
-                    march_tiles(g.nx, g.ny, g.nz, kAdjBand),
-                    ((long long)blockIdx.x - __ldg(block0 + si)) * kMarchWarps +
-                        (threadIdx.x >> 5));
+  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0, adj_set_tiles(g),
+                    (long long)blockIdx.x - __ldg(block0 + si));
 }
 
 namespace {
@@ -370,7 +451,7 @@ __global__ void __launch_bounds__(256) k_edge_adjoint_set(GridSet S,
 }
 
 long long adjoint_grad_blocks(const Grid& g) {
-  return (march_tiles(g.nx, g.ny, g.nz, kAdjBand).tasks + kMarchWarps - 1) / kMarchWarps;
+  return adj_set_tiles(g).tasks;
 }
 long long adjoint_edge_blocks(const Grid& g) { return (g.R * g.wr + 255) / 256; }
 
@@ -380,8 +461,8 @@ void launch_field_adjoint_set(const GridSet& S, const long long* grad_block0,
                               const uint32_t* wv, const float* dverts, const float* dgrad,
                               float* out, cudaStream_t s) {
   if (dgrad && grad_blocks > 0)
-    k_grad_adjoint_set<<<(unsigned)grad_blocks, kMarchWarps * 32, 0, s>>>(S, grad_block0, dgrad,
-                                                                          out);
+    k_grad_adjoint_set<<<(unsigned)grad_blocks, 32, kAdjSmem, s>>>(S, grad_block0, dgrad,
+                                                                               out);
   else
     cudaMemsetAsync(out, 0, (size_t)points * sizeof(float), s);
   if (dverts && edge_blocks > 0)
@@ -393,9 +474,9 @@ void launch_field_adjoint(const Grid& g, const float* f, float iso, const uint32
                           const WordOffsets* o, const float* dverts, const float* dgrad,
                           float* out, int num_sms, cudaStream_t s) {
   if (dgrad) {
-    const MarchTiles mt = march_tiles(g.nx, g.ny, g.nz, kAdjBand);  // tiles of points
-    const long long blocks = (mt.tasks + kMarchWarps - 1) / kMarchWarps;
-    k_grad_adjoint<<<(unsigned)blocks, kMarchWarps * 32, 0, s>>>(g, dgrad, out, mt);
+    const int wave = resident_blocks(k_grad_adjoint, 32, kAdjSmem, num_sms, 1ll << 30);
+    const MarchTiles mt = march_tiles_for(adj_nxw(g), adj_bands(g), g.nz, wave);
+    k_grad_adjoint<<<(unsigned)mt.tasks, 32, kAdjSmem, s>>>(g, dgrad, out, mt);
   } else {
     cudaMemsetAsync(out, 0, (size_t)g.P * sizeof(float), s);
   }

@@ -246,31 +246,50 @@ void launch_thr_emit(const Grid& g, const float* f, const WordOffsets& o, const 
 // z-marching stencil kernels (the adjoint; CellGradient has its own tile
 // constants below): one warp per
 // tile of kMarchCols columns in x (the 32nd lane supplies the +x/-x
-// neighbour column), a band of rows in y and kSeg planes in z, marched
-// along z; kMarchWarps warps (independent tiles) per block.  Band heights
-// and register budgets (blocks per SM) were chosen by timing on GB300.
+// neighbour column), a band of rows in y and a segment of planes in z,
+// marched along z; an adjoint block is one warp.  Band heights and register
+// budgets (blocks per SM) were chosen by timing on GB300.
 constexpr int kMarchCols = 31;
-constexpr int kSeg = 32;
-constexpr int kMarchWarps = 8;
+constexpr int kSeg = 32;            // planes a segment of a grid set's tiles, about
 constexpr int kGradBand = 4;        // cell rows per CellGradient tile
 constexpr int kGradSeg = 16;        // cell planes per CellGradient tile
 constexpr int kGradWarps = 4;       // CellGradient tiles (warps) per block
 constexpr int kGradMinBlocks = 4;
 constexpr int kAdjBand = 8;         // point rows per adjoint tile
-constexpr int kAdjMinBlocks = 3;
+constexpr int kAdjMinBlocks = 28;
 
 struct MarchTiles {
   int nxw, nband, nseg;  // tiles along x, y, z
+  int seg;               // planes a segment (the last may have fewer)
   long long tasks;       // nxw * nband * nseg, x fastest
 };
-// Tiles covering an nx x ny x nz box of cells or points, `band` rows each.
-__host__ __device__ inline MarchTiles march_tiles(int nx, int ny, int nz, int band) {
+__host__ __device__ inline MarchTiles march_tiles(int nxw, int nband, int planes, int nseg) {
   MarchTiles mt;
-  mt.nxw = (nx + kMarchCols - 1) / kMarchCols;
-  mt.nband = (ny + band - 1) / band;
-  mt.nseg = (nz + kSeg - 1) / kSeg;
-  mt.tasks = (long long)mt.nxw * mt.nband * mt.nseg;
+  mt.nxw = nxw;
+  mt.nband = nband;
+  mt.seg = (planes + nseg - 1) / nseg;
+  mt.nseg = (planes + mt.seg - 1) / mt.seg;
+  mt.tasks = (long long)nxw * nband * mt.nseg;
   return mt;
+}
+// The number of segments that wastes least of one grid's adjoint: a wave of
+// `wave` resident tiles runs as long as a segment, which also reads one halo
+// plane and takes about a plane's time to start.  (Cutting the planes of all
+// tiles into equal runs, so that one wave ends together, left neighbouring
+// tiles in different planes and read shared lines twice: 1.5 times the DRAM
+// traffic, 123 -> 162 us at 385 x 321 x 289.)
+inline MarchTiles march_tiles_for(int nxw, int nband, int planes, long long wave) {
+  MarchTiles best{};
+  long long least = -1;
+  for (int nseg = (planes + 63) / 64; nseg <= (planes + 11) / 12; ++nseg) {
+    const MarchTiles mt = march_tiles(nxw, nband, planes, nseg);
+    const long long cost = (mt.tasks + wave - 1) / wave * (mt.seg + 2);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = mt;
+    }
+  }
+  return best;
 }
 
 // dL/dfield from dL/d(merged vertices) (needs the count pass's bits and
