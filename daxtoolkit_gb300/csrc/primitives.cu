@@ -7,7 +7,7 @@
 // to 16 bytes (a dax::Vector3 is 12).
 //
 // Tiles: the float scan works on kPTile elements (256 threads x 16), the sort
-// on kSortTile, the integer scan and the compaction on kSElems:
+// on kSweepTile, the integer scan and the compaction on kSElems:
 //   scan     integers: one pass, each tile's prefix found by a decoupled
 //            look-back over the tiles before it; floats: reduce-then-scan,
 //            tile sums, one block scanning the sums, then each tile scanned
@@ -773,7 +773,7 @@ struct KeyOrder {
 };
 
 // One sweep per digit.  A pass reads every key (and value) once and writes it
-// once: a block takes a tile of kSortTile elements from a ticket counter, ranks
+// once: a block takes a tile of kSweepTile elements from a ticket counter, ranks
 // its keys, publishes its count of every digit, finds how many keys of each
 // digit the earlier tiles hold by looking back over their published counts
 // (thread = digit), and writes the tile out in digit order.  The digits'
@@ -786,13 +786,15 @@ struct KeyOrder {
 // and gathered its values from global memory in digit order: 1.31 ms a pass.
 // Here equal digits are found by eight ballots, values pass through shared
 // memory like the keys, and the look-back replaces histogram and scan:
-// 0.51 ms a pass, against 0.24 ms for its 1.6 GB at the copy bandwidth.  What
+// 0.49 ms a pass, against 0.24 ms for its 1.6 GB at the copy bandwidth.  What
 // is left is about 93 instructions a row of 32 keys and the random shared
-// memory accesses of counters and places (63 % of that pipe); 16 warps of 16
-// keys a thread (64 registers, two blocks an SM) cannot hide all of both.
+// memory accesses of counters and places (63 % of that pipe), which 36 warps
+// of 16 keys a thread cannot hide from one another.  (Finding equal digits by
+// atomicOr of the lanes into a mask a digit, 16 instructions instead of 50 but
+// three more random accesses, took 0.54.)
 //
 // State of (tile, digit), one 32-bit word, zeroed before the pass: 0 nothing
-// yet; count + 1 (count <= kSortTile) the tile's own count; bit 31 | sum the
+// yet; count + 1 (count <= kSweepTile) the tile's own count; bit 31 | sum the
 // count over the tiles up to and including it (n < 2^31).
 // Tickets go out in tile order, so a wait is only ever on a block that is
 // running.  The wait is bounded all the same, and a thread whose wait runs out
@@ -802,9 +804,20 @@ constexpr int kSortThreads = 512;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kSortWarps = kSortThreads / 32;
+
+// A sweep's blocks are smaller than the one that sorts alone, so that more of
+// them, in different phases, share an SM: three of 4-byte keys with up to one
+// word of values, two otherwise (by registers and shared memory).  100 M int32
+// pairs: 2.14 ms with three of 384 threads, the same with two of 512, 2.36 with
+// two of 384; 30 M int64 pairs: 1.72, 2.18 (one block fits) and 1.72 ms.
+constexpr int kSweepThreads = 384;
+constexpr int kSweepTile = kSweepThreads * kSortItems;
+constexpr int kSweepWarps = kSweepThreads / 32;
+template <typename U, int VW>
+constexpr int kSweepBlocks = sizeof(U) == 4 && VW <= 1 ? 3 : 2;
 constexpr uint32_t kSortInc = 0x80000000u;
 
-int sort_tiles(long long n) { return (int)((n + kSortTile - 1) / kSortTile); }
+int sort_tiles(long long n) { return (int)((n + kSweepTile - 1) / kSweepTile); }
 
 // Lanes whose digit (bits shift .. shift + 7 of the key) equals this lane's:
 // a ballot per bit.
@@ -823,11 +836,20 @@ __device__ __forceinline__ unsigned equal_digits(U key, int shift) {
   return peers;
 }
 
+// Places in a tile, below 2^16: two a register.
+struct Places {
+  uint32_t p[kSortItems / 2];
+  __device__ __forceinline__ uint32_t get(int e) const { return (p[e / 2] >> (16 * (e & 1))) & 0xffffu; }
+  __device__ __forceinline__ void set(int e, uint32_t v) {
+    p[e / 2] = (e & 1) ? __byte_perm(p[e / 2], v, 0x5410) : __byte_perm(p[e / 2], v, 0x3254);
+  }
+};
+
 // Ranks a warp's keys (rows of 32, in row then lane order) among its equal
 // digits; cnt: the warp's 256 counters, zero before, its digit counts after.
 // FULL: every row holds 32 keys; else the first `count` places do.
 template <bool FULL, typename U>
-__device__ __forceinline__ void warp_rank(const U (&key)[kSortItems], uint32_t (&rank)[kSortItems],
+__device__ __forceinline__ void warp_rank(const U (&key)[kSortItems], Places& rank,
                                           int shift, int count, int lane, uint32_t* cnt) {
   const unsigned lt = (1u << lane) - 1u;
   constexpr int kG = 4;  // rows whose masks, which do not depend on one another, come first
@@ -850,7 +872,7 @@ __device__ __forceinline__ void warp_rank(const U (&key)[kSortItems], uint32_t (
         __syncwarp();
         if (ok && below == 0u) *c = before + __popc(peers[g]);
         __syncwarp();
-        rank[e0 + g] = before + below;
+        rank.set(e0 + g, before + below);
       }
   }
 }
@@ -858,12 +880,13 @@ __device__ __forceinline__ void warp_rank(const U (&key)[kSortItems], uint32_t (
 // Turns the warps' digit counts s_cnt[warp][256] into each (warp, digit)'s
 // first place in the tile sorted by digit; threads 0..255 return their
 // digit's count and, in *start, its first place.  s_warp: 8 words.
+template <int WARPS>
 __device__ __forceinline__ uint32_t place_digits(uint32_t* s_cnt, uint32_t* s_warp, uint32_t* start) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t tot = 0, x = 0;
   if (tid < 256) {
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       const uint32_t c = s_cnt[w * 256 + tid];
       s_cnt[w * 256 + tid] = tot;
       tot += c;
@@ -882,7 +905,7 @@ __device__ __forceinline__ uint32_t place_digits(uint32_t* s_cnt, uint32_t* s_wa
     for (int w = 0; w < warp; ++w) x += s_warp[w];
     *start = x;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) s_cnt[w * 256 + tid] += x;
+    for (int w = 0; w < WARPS; ++w) s_cnt[w * 256 + tid] += x;
   }
   return tot;
 }
@@ -934,8 +957,8 @@ void opt_in_smem(const void* kernel, size_t smem, int* done) {
 template <typename U>
 __device__ __forceinline__ uint32_t count_digit(const U* kin, long long n, int tile, int shift,
                                              unsigned d, KeyOrder<U> ord) {
-  const long long b = (long long)tile * kSortTile;
-  const long long e = b + kSortTile < n ? b + kSortTile : n;
+  const long long b = (long long)tile * kSweepTile;
+  const long long e = b + kSweepTile < n ? b + kSweepTile : n;
   uint32_t c = 0;
 #pragma unroll 1
   for (long long i = b; i < e; ++i) c += ((unsigned)(ord.load(kin[i]) >> shift) & 255u) == d;
@@ -981,12 +1004,12 @@ __device__ __forceinline__ uint32_t digit_look_back(const uint32_t* state, int t
 
 template <typename U>
 constexpr size_t sweep_smem(int vwords) {
-  return (size_t)kSortTile * sizeof(U) + (vwords ? (size_t)kSortTile * 4 : 0) +
-         (size_t)kSortWarps * 256 * 4 + 256 * 4 + 16 * 4;
+  return (size_t)kSweepTile * sizeof(U) + (vwords ? (size_t)kSweepTile * 4 : 0) +
+         (size_t)kSweepWarps * 256 * 4 + 256 * 4 + 16 * 4;
 }
 
 // One tile of a pass.  VW: 32-bit words a value (0: keys only); FULL: the
-// tile holds kSortTile elements.
+// tile holds kSweepTile elements.
 template <typename U, int VW, bool FULL>
 __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restrict__ kout,
                                            const uint32_t* __restrict__ vin,
@@ -996,12 +1019,12 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
                                            const KeyOrder<U>& ord, U* s_key, uint32_t* s_val,
                                            uint32_t* s_cnt, uint32_t* s_dst, uint32_t* s_warp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long tb = (long long)tile * kSortTile;
-  const int valid = FULL ? kSortTile : (int)(n - tb);
+  const long long tb = (long long)tile * kSweepTile;
+  const int valid = FULL ? kSweepTile : (int)(n - tb);
   const int l0 = warp * (kSortItems * 32) + lane;  // the thread's first element of the tile
   const U* kt = kin + tb + l0;
   U key[kSortItems];
-  uint32_t rank[kSortItems];
+  Places rank;
 #pragma unroll
   for (int e = 0; e < kSortItems; ++e)
     key[e] = FULL || l0 + 32 * e < valid ? __ldcs(kt + 32 * e) : (U)0;
@@ -1011,15 +1034,16 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
   warp_rank<FULL>(key, rank, shift, valid - (l0 - lane), lane, cnt);
   __syncthreads();
   uint32_t lstart = 0;
-  const uint32_t tot = place_digits(s_cnt, s_warp, &lstart);
+  const uint32_t tot = place_digits<kSweepWarps>(s_cnt, s_warp, &lstart);
   uint32_t* mine = state + (long long)tile * 256 + tid;
   if (tid < 256) st_relaxed(mine, tile == 0 ? kSortInc | tot : tot + 1u);
   __syncthreads();
 #pragma unroll
   for (int e = 0; e < kSortItems; ++e)
     if (FULL || l0 + 32 * e < valid) {
-      rank[e] += cnt[(unsigned)(key[e] >> shift) & 255u];  // its place in the tile
-      s_key[rank[e]] = key[e];
+      const uint32_t at = rank.get(e) + cnt[(unsigned)(key[e] >> shift) & 255u];  // its place in the tile
+      rank.set(e, at);
+      s_key[at] = key[e];
     }
   uint32_t v[VW ? kSortItems : 1];
   auto load_values = [&](int q) {
@@ -1031,7 +1055,7 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
   auto place_values = [&]() {
 #pragma unroll
     for (int e = 0; e < kSortItems; ++e)
-      if (FULL || l0 + 32 * e < valid) s_val[rank[e]] = v[e];
+      if (FULL || l0 + 32 * e < valid) s_val[rank.get(e)] = v[e];
   };
   if constexpr (VW > 0) load_values(0);  // in flight during the look-back
   if (tid < 256) {
@@ -1055,7 +1079,7 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
   __syncthreads();
 #pragma unroll
   for (int e = 0; e < kSortItems; ++e) {
-    const int j = tid + e * kSortThreads;
+    const int j = tid + e * kSweepThreads;
     if (FULL || j < valid) {
       const U k = s_key[j];
       const uint32_t at = s_dst[(unsigned)(k >> shift) & 255u] + j;
@@ -1072,7 +1096,7 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
       __syncthreads();
 #pragma unroll
       for (int e = 0; e < kSortItems; ++e) {
-        const int j = tid + e * kSortThreads;
+        const int j = tid + e * kSweepThreads;
         if (FULL || j < valid) {
           const uint32_t at = s_dst[(unsigned)(s_key[j] >> shift) & 255u] + j;
           vout[(long long)at * VW + q] = s_val[j];
@@ -1084,24 +1108,24 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
 
 // One pass: hist: the digits' counts over all keys.
 template <typename U, int VW>
-__global__ void __launch_bounds__(kSortThreads, 2)
+__global__ void __launch_bounds__(kSweepThreads, (kSweepBlocks<U, VW>))
     k_radix_sweep(const U* __restrict__ kin, U* __restrict__ kout, const uint32_t* __restrict__ vin,
                   uint32_t* __restrict__ vout, long long n, int shift,
                   const uint32_t* __restrict__ hist, uint32_t* __restrict__ state,
                   unsigned* __restrict__ ticket, KeyOrder<U> ord) {
   extern __shared__ unsigned long long s_dyn[];
-  U* s_key = reinterpret_cast<U*>(s_dyn);                            // [kSortTile]
-  uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + kSortTile);  // [kSortTile] if VW
-  uint32_t* s_cnt = s_val + (VW ? kSortTile : 0);                    // [kSortWarps][256]
-  uint32_t* s_dst = s_cnt + kSortWarps * 256;  // [256] global place of the run - its local start
+  U* s_key = reinterpret_cast<U*>(s_dyn);                            // [kSweepTile]
+  uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + kSweepTile);  // [kSweepTile] if VW
+  uint32_t* s_cnt = s_val + (VW ? kSweepTile : 0);                    // [kSweepWarps][256]
+  uint32_t* s_dst = s_cnt + kSweepWarps * 256;  // [256] global place of the run - its local start
   uint32_t* s_warp = s_dst + 256;              // [16]
   __shared__ int s_tile;
   if (threadIdx.x == 0) s_tile = (int)atomicAdd(ticket, 1u);
-  for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads) s_cnt[i] = 0;
+  for (int i = threadIdx.x; i < kSweepWarps * 256; i += kSweepThreads) s_cnt[i] = 0;
   __syncthreads();
   const int tile = s_tile;
-  if ((long long)tile * kSortTile >= n) return;
-  if ((long long)(tile + 1) * kSortTile <= n)
+  if ((long long)tile * kSweepTile >= n) return;
+  if ((long long)(tile + 1) * kSweepTile <= n)
     sweep_tile<U, VW, true>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, s_key, s_val,
                             s_cnt, s_dst, s_warp);
   else
@@ -1131,7 +1155,7 @@ __global__ void __launch_bounds__(kSortThreads, 1)
   const int count = min(n - w0, rows * 32);  // the warp's keys (<= 0: none)
   uint32_t* cnt = s_cnt + warp * 256;
   U key[kSortItems];
-  uint32_t rank[kSortItems];
+  Places rank;
   uint16_t src[kSortItems];
 #pragma unroll
   for (int e = 0; e < kSortItems; ++e) {
@@ -1158,12 +1182,12 @@ __global__ void __launch_bounds__(kSortThreads, 1)
     warp_rank<false>(key, rank, shift, count, lane, cnt);
     __syncthreads();
     uint32_t start;
-    place_digits(s_cnt, s_warp, &start);
+    place_digits<kSortWarps>(s_cnt, s_warp, &start);
     __syncthreads();
 #pragma unroll
     for (int e = 0; e < kSortItems; ++e) {
       if (e < rows && w0 + 32 * e + lane < n) {
-        const uint32_t at = cnt[(unsigned)(key[e] >> shift) & 255u] + rank[e];
+        const uint32_t at = cnt[(unsigned)(key[e] >> shift) & 255u] + rank.get(e);
         s_key[at] = key[e];
         s_src[at] = src[e];
       }
@@ -1414,7 +1438,7 @@ void launch_sweep(const U* kin, U* kout, const uint32_t* vin, uint32_t* vout, lo
   static int opted[64] = {};
   constexpr size_t smem = sweep_smem<U>(VW);
   opt_in_smem((const void*)k_radix_sweep<U, VW>, smem, opted);
-  k_radix_sweep<U, VW><<<sort_tiles(n), kSortThreads, smem, s>>>(kin, kout, vin, vout, n, shift,
+  k_radix_sweep<U, VW><<<sort_tiles(n), kSweepThreads, smem, s>>>(kin, kout, vin, vout, n, shift,
                                                                 hist, state, ticket, ord);
 }
 
@@ -1425,8 +1449,8 @@ void launch_sweep(const U* kin, U* kout, const uint32_t* vin, uint32_t* vout, lo
 // Up to kSortTile elements are one launch of one block.  Longer arrays keep
 // the tile states, the digit counts and the tickets in the scratch's
 // histogram section: 1 KB per 4096 elements, of which the states take 1 KB
-// per kSortTile = 8192; the counts of as many passes as fit beside them
-// (all, from 64 K elements) are taken at a time.
+// per kSweepTile = 6144; the counts of as many passes as fit beside them
+// (all, from 94 K elements) are taken at a time.
 template <typename U>
 void radix_sort(U* keys, uint32_t* vals, int vwords, long long n, int kind, bool desc,
                 char* scratch, int num_sms, cudaStream_t s, int passes = (int)sizeof(U),
