@@ -109,6 +109,11 @@ __device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_warp, uns
 // Warp w of a tile takes the kMtChunk consecutive cells of chunk 8 * tile + w
 // (lanes interleaved, so every load of ids is 512 contiguous bytes); the
 // chunk's and the tile's triangle totals are stored.
+//
+// 83 million cells take 280 us, 1.33 GB of connectivity at 4.7 TB/s: the
+// gathers of a row of 32 cells touch 4 to 8 lines each, which L1 looks up one
+// at a time.  (The ids of two, four or eight cells loaded ahead of their
+// gathers took 310, 300 and 400 us.)
 template <bool VEC>
 __global__ void __launch_bounds__(kMtThreads) k_mt_count(const int32_t* __restrict__ conn,
                                                          long long C,
@@ -159,36 +164,42 @@ __global__ void __launch_bounds__(kMtThreads) k_mt_count(const int32_t* __restri
 
 // One block: exclusive offsets of the tile totals (tile_off[tiles] = T) and
 // the total into Info; more than 2^31 - 1 vertex records is an overflow.
-// Thread t sums its own contiguous run of tiles, the block scans the 1024
-// run totals, then every thread writes its run's offsets.
+// Warp w sums its own contiguous run of tiles, 32 at a time, the block scans
+// the 32 run totals, then every warp scans its run.  (A run a thread, whose
+// loads lay 80 bytes apart, took 19 us for 20 thousand tiles; 12 now.)
 __global__ void __launch_bounds__(1024) k_mt_tile_scan(const unsigned* __restrict__ tile_tot,
                                                        int tiles,
                                                        unsigned long long* __restrict__ tile_off,
                                                        Info* info) {
   __shared__ unsigned long long s_warp[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int per = (tiles + 1023) / 1024;
-  const int b = threadIdx.x * per, e = min(b + per, tiles);
+  const int per = (tiles + 1023) / 1024 * 32;  // tiles a warp
+  const int b = wid * per, e = min(b + per, tiles);
   unsigned long long v = 0;
-  for (int i = b; i < e; ++i) v += tile_tot[i];
-  unsigned long long x = v;
+#pragma unroll 4
+  for (int i = b + lane; i < e; i += 32) v += tile_tot[i];
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned long long y = __shfl_up_sync(kFull, x, d);
-    if (lane >= d) x += y;
-  }
-  if (lane == 31) s_warp[wid] = x;
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);
+  if (lane == 0) s_warp[wid] = v;
   __syncthreads();
-  unsigned long long before = 0, all = 0;
+  unsigned long long run = 0, all = 0;
   for (int w = 0; w < 32; ++w) {
     const unsigned long long t = s_warp[w];
-    before += w < wid ? t : 0ull;
+    run += w < wid ? t : 0ull;
     all += t;
   }
-  unsigned long long run = before + x - v;
-  for (int i = b; i < e; ++i) {
-    tile_off[i] = run;
-    run += tile_tot[i];
+#pragma unroll 4
+  for (int i0 = b; i0 < e; i0 += 32) {
+    const int i = i0 + lane;
+    const unsigned long long t = i < e ? tile_tot[i] : 0u;
+    unsigned long long x = t;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const unsigned long long y = __shfl_up_sync(kFull, x, d);
+      if (lane >= d) x += y;
+    }
+    if (i < e) tile_off[i] = run + x - t;
+    run += __shfl_sync(kFull, x, 31);
   }
   if (threadIdx.x == 0) {
     tile_off[tiles] = all;
@@ -358,7 +369,11 @@ __device__ __forceinline__ bool merge_header_ok(const MtMergeHeader* h, long lon
          n * sizeof(U) <= mbytes - h->uniq;
 }
 
-// conn[r] = LowerBounds(unique keys, key of record r).
+// conn[r] = LowerBounds(unique keys, key of record r).  The first ten steps of
+// the search run over 1023 of the keys, evenly spaced, that each block holds in
+// shared memory: all 21 steps through L2 took 41 us for 2 M records of 1 M
+// keys, now 32.
+constexpr int kMtSamples = 1023;
 template <typename U>
 __global__ void __launch_bounds__(256) k_mt_merged_conn(const char* __restrict__ m,
                                                         unsigned long long mbytes, Info* info,
@@ -379,10 +394,20 @@ __global__ void __launch_bounds__(256) k_mt_merged_conn(const char* __restrict__
   const U* __restrict__ keys = reinterpret_cast<const U*>(m + hdr->keys);
   const U* __restrict__ uniq = reinterpret_cast<const U*>(m + hdr->uniq);
   const long long n = 3 * T;
+  __shared__ U s_key[kMtSamples];  // key at (i + 1) V / 1024
+  for (int i = threadIdx.x; i < kMtSamples; i += blockDim.x) {
+    const long long at = (i + 1) * V / (kMtSamples + 1);
+    s_key[i] = at < V ? uniq[at] : ~(U)0;
+  }
+  __syncthreads();
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (long long)gridDim.x * blockDim.x) {
     const U k = keys[r];
-    long long lo = 0, hi = V;
+    int below = 0;  // samples less than k
+#pragma unroll
+    for (int step = (kMtSamples + 1) / 2; step > 0; step >>= 1)
+      if (s_key[below + step - 1] < k) below += step;
+    long long lo = below * V / (kMtSamples + 1), hi = (below + 1) * V / (kMtSamples + 1);
     while (lo < hi) {
       const long long mid = (lo + hi) >> 1;
       if (__ldg(uniq + mid) < k) lo = mid + 1;
