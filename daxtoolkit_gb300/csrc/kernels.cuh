@@ -202,7 +202,7 @@ void launch_mc_scan_slab(const GridSet& S, const uint32_t* bits, const WordOffse
 // The emit of the active words act[slab_act[0] .. slab_act[1]) of row words
 // [word_begin, word_end), capacity-checked at the offsets of range_end
 // (range_end < 0: every active word, after a complete count pass).
-// Warps take `batch` active words at a time from *ticket (reset to 0 with
+// Warps take up to `batch` active words at a time from *ticket (reset to 0 with
 // *done by the launch's last block).  kEmitBatch: the batch of a whole-grid
 // emit.
 constexpr int kEmitBatch = 16;

@@ -628,6 +628,7 @@ enum EmitField {
   kFields = 31
 };
 constexpr int kEmitWarps = 8;
+constexpr int kEmitLeast = 4;
 
 __device__ __forceinline__ uint32_t window(const uint32_t* st, int f, int s) { return st[f * 32 + s]; }
 
@@ -703,11 +704,21 @@ __device__ __forceinline__ void cell_edge_ids(const uint32_t* st, int s, int q, 
   ids[11 * 32 + lane] = R[1] + x[1] + y[1];           // row 1, q,     z
 }
 
-// A warp takes `batch` (1..32) active words at a time from the counter
-// *ticket; the last block to finish resets *ticket and *done.  Smaller
-// batches shorten each warp's chain of dependent steps (the kernel's
-// duration when its words are few), larger ones share each step over more
-// words.
+// A warp takes up to `batch` (1..32) active words at a time from the counter
+// *ticket; the last block to finish resets *ticket and *done.  While there is
+// more than one round of them left, a batch is half of a warp's share of what
+// is left, so that the rounds shrink and the warps end together; then it is the
+// share, down to kEmitLeast words.  (Merged, a round of up to 20 words a warp
+// costs less than two smaller ones: 19 against 23 us on a slice of 383 x 405 x
+// 331.  Unmerged, words differ more and the line lies at 6: 79 against 100 us
+// on the Mandelbulb.  Fixed batches of 16: 24 -> 14 us for the 128^3 benchmark,
+// 27 -> 20 for 301 x 257 x 199, 45 -> 43 at 512^3.)
+//
+// Unmerged, the vertices of a chunk of 32 cells are dealt to the lanes in
+// output order: a lane looping over its own cell's triangles kept 16 of 32
+// lanes busy and stored 36 bytes apart, 133 us for the 4.6 M vertices of the
+// 201^3 Mandelbulb, now 79.  (Merged, dealing the ids the same way was slower,
+// 49 against 43 us at 512^3: its triangles are three loads each.)
 // range_end < 0: every active word, after a complete count pass.
 // range_end >= 0 (one slab of the pipelined marching cubes, one grid): the
 // active words act[slab_act[0] .. slab_act[1]), which lie below row word
@@ -737,6 +748,11 @@ __global__ void __launch_bounds__(kEmitWarps * 32, 4) k_mc_emit(GridSet S,
   __shared__ int s_pre[kEmitWarps][33];    // active cells before word s
   __shared__ int s_ppre[kEmitWarps][33];   // owner points (points with owned edges) before word s
   __shared__ uint32_t s_ids[kEmitWarps][MERGE ? 12 * 32 : 1];  // a cell's 12 edge ids per lane
+  // unmerged: the chunk's cells (case word, word << 5 | bit) and, per triangle
+  // of the chunk, its cell and its place in the cell (cell | place << 5)
+  __shared__ uint64_t s_cell[MERGE ? 1 : kEmitWarps][32];
+  __shared__ uint16_t s_at[MERGE ? 1 : kEmitWarps][32];
+  __shared__ unsigned char s_tri[MERGE ? 1 : kEmitWarps][5 * 32];
   __shared__ long long s_keys[kStagedSlots];
   s_case[threadIdx.x] = kMcCase[threadIdx.x];
   if (threadIdx.x < 12) s_edge[threadIdx.x] = kEdgeOwner[threadIdx.x];
@@ -762,17 +778,21 @@ __global__ void __launch_bounds__(kEmitWarps * 32, 4) k_mc_emit(GridSet S,
   int* pre = s_pre[wib];
   int* ppre = s_ppre[wib];
   uint32_t* ids = s_ids[wib];
-  while (true) {
+  const long long warps = (long long)gridDim.x * kEmitWarps;
+  for (long long left = A - A0; left > 0;) {
     // the next batch of active words, taken dynamically (batches differ
-    // widely in cost)
+    // widely in cost); its size from what was left at the last one
+    const long long each = (left + warps - 1) / warps;
+    const int take = (int)min((long long)batch, each > (MERGE ? 20 : 6) ? each / 2 : max(each, (long long)kEmitLeast));
     long long a0 = 0;
-    if (lane == 0) a0 = A0 + (long long)batch * atomicAdd(ticket, 1u);
+    if (lane == 0) a0 = A0 + (long long)atomicAdd(ticket, (unsigned)take);
     a0 = __shfl_sync(kFull, a0, 0);
+    left = A - a0 - take;
     if (a0 >= A) break;
     // ---- lane = word: gather the word's bits, masks and offsets ----------
     uint32_t am = 0, t0 = 0;
     int np = 0;
-    if (lane < batch && a0 + lane < A) {
+    if (lane < take && a0 + lane < A) {
       const uint32_t gw = __ldg(o.act + a0 + lane);
       t0 = __ldg(o.wt + gw);
       int si, m;
@@ -892,34 +912,38 @@ __global__ void __launch_bounds__(kEmitWarps * 32, 4) k_mc_emit(GridSet S,
       }
       int chunk_tri;
       const int ex = warp_exclusive(nt, lane, &chunk_tri);
-      if (nt > 0) {
-        const long long tri0 = tri_base + ex;
-        const GridSlot& sl = S.count == 1 ? S.one : S.slots[window(st, kFSlot, s)];
-        // first vertex of this grid in the concatenated output (0 for one grid)
-        const long long vbase0 =
-            S.count == 1 ? 0 : (MERGE ? word_v(o, sl.rw0) : 3 * word_t(o, sl.rw0));
-        if (MERGE) {
+      if constexpr (MERGE) {
+        if (nt > 0) {
+          const GridSlot& sl = S.count == 1 ? S.one : S.slots[window(st, kFSlot, s)];
+          // first vertex of this grid in the concatenated output (0 for one grid)
+          const long long vbase0 = S.count == 1 ? 0 : word_v(o, sl.rw0);
           cell_edge_ids(st, s, q, ids, lane);
           for (int t = 0; t < nt; ++t) {
-            int32_t* out = conn + 3 * (tri0 + t);
+            int32_t* out = conn + 3 * (tri_base + ex + t);
 #pragma unroll
             for (int corner = 0; corner < 3; ++corner)
               out[corner] = (int32_t)((long long)ids[mc_edge(cw, 3 * t + corner) * 32 + lane] - vbase0);
           }
-        } else {
-          const int i = (int)window(st, kFI0, s) + q, j = (int)window(st, kFJ, s),
-                    k = (int)window(st, kFK, s);
-          for (int t = 0; t < nt; ++t) {
-#pragma unroll
-            for (int corner = 0; corner < 3; ++corner) {
-              const int info_e = s_edge[mc_edge(cw, 3 * t + corner)];
-              const int di = info_e & 1, dj = (info_e >> 1) & 1, dk = (info_e >> 2) & 1;
-              const long long vid = 3 * (tri0 + t) + corner;
-              conn[vid] = (int32_t)(vid - vbase0);
-              emit_vertex(sl, i + di, j + dj, k + dk, info_e >> 3, vid, verts, ra, rb, rw);
-            }
-          }
         }
+      } else {
+        s_cell[wib][lane] = cw;
+        s_at[wib][lane] = (uint16_t)(s << 5 | q);
+        for (int t = 0; t < nt; ++t) s_tri[wib][ex + t] = (unsigned char)(lane | t << 5);
+        __syncwarp();
+        for (int v = lane; v < 3 * chunk_tri; v += 32) {
+          const int tri = v / 3, r = v - 3 * tri;
+          const int cell = s_tri[wib][tri] & 31, place = s_tri[wib][tri] >> 5;
+          const int at = s_at[wib][cell], w = at >> 5;
+          const GridSlot& sl = S.count == 1 ? S.one : S.slots[window(st, kFSlot, w)];
+          const long long vbase0 = S.count == 1 ? 0 : 3 * word_t(o, sl.rw0);
+          const int info_e = s_edge[mc_edge(s_cell[wib][cell], 3 * place + r)];
+          const int di = info_e & 1, dj = (info_e >> 1) & 1, dk = (info_e >> 2) & 1;
+          const long long vid = 3 * tri_base + v;
+          conn[vid] = (int32_t)(vid - vbase0);
+          emit_vertex(sl, (int)window(st, kFI0, w) + (at & 31) + di, (int)window(st, kFJ, w) + dj,
+                      (int)window(st, kFK, w) + dk, info_e >> 3, vid, verts, ra, rb, rw);
+        }
+        __syncwarp();
       }
       tri_base += chunk_tri;
     }

@@ -13,11 +13,11 @@ def _field(dims, seed):
     return np.random.default_rng(seed).uniform(0, 1, size=dims[0] * dims[1] * dims[2]).astype(np.float32)
 
 
-def _check(out, dims, f, iso):
+def _check(out, dims, f, iso, merge=True):
     import oracle
     O = oracle.Oracle("port")
     og = oracle.make_grid(dims)
-    ref = O.mc_generate(og, f, iso, O.mc_count(og, f, iso)[0], merge=True)
+    ref = O.mc_generate(og, f, iso, O.mc_count(og, f, iso)[0], merge=merge)
     assert np.array_equal(out[1], ref["conn"])
     assert np.array_equal(out[0].view(np.uint32), ref["verts"].view(np.uint32))
 
@@ -43,3 +43,26 @@ def test_counts_of_a_set(sets):
     verts, conn = verts.cpu().numpy(), conn.cpu().numpy()
     for i in list(range(0, len(sets), 1 + len(sets) // 12)) + [len(sets) - 1]:
         _check((verts[vert[i]:vert[i + 1]], conn[tri[i]:tri[i + 1]]), sets[i], fields[i], 0.5)
+
+
+@pytest.mark.parametrize("iso", [0.5, 0.995])
+@pytest.mark.parametrize("dims", SHAPES)
+def test_unmerged_vertices_of_one_grid(dims, iso):
+    import torch
+    from daxtoolkit_gb300 import cont
+    f = _field(dims, dims[0] + 1)
+    out = cont.marching_cubes(cont.UniformGrid(dims), torch.from_numpy(f).cuda(), iso, merge=False)
+    _check((out["verts"].cpu().numpy(), out["conn"].cpu().numpy()), dims, f, iso, merge=False)
+
+
+def test_unmerged_vertices_of_a_set():
+    import torch
+    from daxtoolkit_gb300 import cont
+    sets = SHAPES + [(5, 4, 4)] * 40
+    fields = [_field(d, i) for i, d in enumerate(sets)]
+    batch = cont.MarchingCubesBatch([cont.UniformGrid(d) for d in sets], [torch.from_numpy(f).cuda() for f in fields],
+                                    [0.5] * len(sets))
+    verts, conn, tri, _ = batch.run(merge=False)
+    verts, conn = verts.cpu().numpy(), conn.cpu().numpy()
+    for i, d in enumerate(sets):
+        _check((verts[3 * tri[i]:3 * tri[i + 1]], conn[tri[i]:tri[i + 1]]), d, fields[i], 0.5, merge=False)
