@@ -105,38 +105,71 @@ __global__ void __launch_bounds__(256) k_mandelbulb_field(Grid g, float* __restr
 // (VectorAnalysis.h:182-201, 227-232; RSqrt is 1 / Sqrt off the GPU), its
 // colour the cool-warm entry (int)(257 * clamp(|dot(p, (0.09, 0.09, 0.9))|,
 // 0, 0.9999)) (CoolWarmColorMap.h:38-45) with alpha 255.
+__device__ __forceinline__ float3 triangle_normal(const float* c) {
+  const float ax = __fsub_rn(c[3], c[0]), ay = __fsub_rn(c[4], c[1]), az = __fsub_rn(c[5], c[2]);
+  const float bx = __fsub_rn(c[6], c[0]), by = __fsub_rn(c[7], c[1]), bz = __fsub_rn(c[8], c[2]);
+  const float xx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
+  const float xy = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
+  const float xz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(magsq3(xx, xy, xz)));
+  return make_float3(__fmul_rn(r, xx), __fmul_rn(r, xy), __fmul_rn(r, xz));
+}
+
+__device__ __forceinline__ uchar4 point_color(const float* p, const unsigned char* map) {
+  float s = __fadd_rn(__fadd_rn(__fmul_rn(p[0], 0.09f), __fmul_rn(p[1], 0.09f)), __fmul_rn(p[2], 0.9f));
+  s = fminf(0.9999f, fmaxf(0.0f, fabsf(s)));
+  const int idx = (int)__fmul_rn(257.0f, s);
+  return make_uchar4(map[3 * idx + 0], map[3 * idx + 1], map[3 * idx + 2], 255);
+}
+
+// Bound by HBM, 28 bytes a point.  A warp takes 32 triangles, 1152 consecutive
+// bytes in and out, through shared memory, lane = triangle: every normal is
+// computed once and every access of global memory covers 128 bytes.  (Lane =
+// point, each computing its triangle's normal from nine strided loads: 44 us
+// for 4.6 M points, 35 now.)  nv is a multiple of 3.
 __global__ void __launch_bounds__(256) k_colors_and_norms(const float* __restrict__ verts,
                                                           long long nv, float* __restrict__ norms,
                                                           uint8_t* __restrict__ colors) {
   __shared__ unsigned char s_map[3 * DAX_GB300_COOLWARM_ENTRIES];
+  __shared__ float s_buf[8][9 * 32];
+  __shared__ uchar4 s_color[8][3 * 32];
   for (int t = threadIdx.x; t < 3 * DAX_GB300_COOLWARM_ENTRIES; t += blockDim.x)
     s_map[t] = c_coolwarm[t];
   __syncthreads();
-  for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < nv;
-       v += (long long)gridDim.x * blockDim.x) {
-    const float* c0 = verts + 3 * (3 * (v / 3));
-    const float ax = __fsub_rn(c0[3], c0[0]), ay = __fsub_rn(c0[4], c0[1]),
-                az = __fsub_rn(c0[5], c0[2]);
-    const float bx = __fsub_rn(c0[6], c0[0]), by = __fsub_rn(c0[7], c0[1]),
-                bz = __fsub_rn(c0[8], c0[2]);
-    const float xx = __fsub_rn(__fmul_rn(ay, bz), __fmul_rn(az, by));
-    const float xy = __fsub_rn(__fmul_rn(az, bx), __fmul_rn(ax, bz));
-    const float xz = __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(magsq3(xx, xy, xz)));
-    norms[3 * v + 0] = __fmul_rn(r, xx);
-    norms[3 * v + 1] = __fmul_rn(r, xy);
-    norms[3 * v + 2] = __fmul_rn(r, xz);
-    const float* p = verts + 3 * v;
-    float s = __fadd_rn(__fadd_rn(__fmul_rn(p[0], 0.09f), __fmul_rn(p[1], 0.09f)),
-                        __fmul_rn(p[2], 0.9f));
-    s = fminf(0.9999f, fmaxf(0.0f, fabsf(s)));
-    const int idx = (int)__fmul_rn(257.0f, s);
-    uchar4 c;
-    c.x = s_map[3 * idx + 0];
-    c.y = s_map[3 * idx + 1];
-    c.z = s_map[3 * idx + 2];
-    c.w = 255;
-    reinterpret_cast<uchar4*>(colors)[v] = c;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* const buf = s_buf[warp];
+  uchar4* const color = s_color[warp];
+  const long long T = nv / 3, step = (long long)gridDim.x * 8 * 32;
+  for (long long t0 = ((long long)blockIdx.x * 8 + warp) * 32; t0 < T; t0 += step) {
+    const int n = (int)min(32ll, T - t0);  // triangles
+    const float* in = verts + 9 * t0;
+    float* out = norms + 9 * t0;
+    uchar4* cout = reinterpret_cast<uchar4*>(colors) + 3 * t0;
+#pragma unroll
+    for (int e = 0; e < 9; ++e)
+      if (32 * e + lane < 9 * n) buf[32 * e + lane] = __ldg(in + 32 * e + lane);
+    __syncwarp();
+    float c[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) c[e] = buf[9 * lane + e];
+    const float3 x = triangle_normal(c);
+    if (lane < n) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        color[3 * lane + q] = point_color(c + 3 * q, s_map);
+        buf[9 * lane + 3 * q] = x.x;
+        buf[9 * lane + 3 * q + 1] = x.y;
+        buf[9 * lane + 3 * q + 2] = x.z;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 9; ++e)
+      if (32 * e + lane < 9 * n) out[32 * e + lane] = buf[32 * e + lane];
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+      if (32 * e + lane < 3 * n) cout[32 * e + lane] = color[32 * e + lane];
+    __syncwarp();
   }
 }
 
@@ -147,7 +180,7 @@ void launch_mandelbulb_field(const Grid& g, float* out, int num_sms, cudaStream_
 
 void launch_colors_and_norms(const float* verts, long long nv, float* norms, uint8_t* colors,
                              int num_sms, cudaStream_t s) {
-  const int b = resident_blocks(k_colors_and_norms, 256, 0, num_sms, (nv + 255) / 256);
+  const int b = resident_blocks(k_colors_and_norms, 256, 0, num_sms, (nv / 3 + 255) / 256);
   k_colors_and_norms<<<b, 256, 0, s>>>(verts, nv, norms, colors);
 }
 
