@@ -13,7 +13,7 @@
 // K2b (k_word_scan, shared with marching cubes): per-word exclusive offsets
 //     wt (kept cells) and wv (used points), the compacted list act of the
 //     words with either, and the totals.
-// K3 (k_thr_emit): a warp loads 32 active words at once (lane = word),
+// K3 (k_thr_emit): a warp loads kThrBatch active words at once (lane = word),
 //     starts the copies of the field values of all their used points into
 //     shared memory (cp.async, one wait per batch), then walks the words
 //     with lane = bit: the word's used points (coordinates and field:
@@ -206,6 +206,11 @@ void launch_thr_count(const Grid& g, const uint32_t* bits, uint32_t* kept, uint3
   launch_pdl(k_thr_used, (unsigned)b2, 256u, 0, s, g, kept, used, wc, tile_tot, tiles);
 }
 
+// Words a warp of the emit takes at a time.  Small batches even the warps out:
+// 133, 139, 143 and 145 us with 8, 16, 24 and 32 at 512^3, 11 to 16 us at 200 x
+// 180 x 150.
+constexpr int kThrBatch = 8;
+
 // Per active word, what the emit loop needs: its masks and offsets, and for
 // kept cells the used masks and offsets of corner rows q = dj + 2 dk
 // (q = 1..3) at word m, and the first used-point offsets of rows q = 0..3 at
@@ -221,7 +226,7 @@ struct ThrWord {
 // latency of each word's chain: stores of whole sectors (a cell is one 32-byte
 // store, a word's coordinates leave through shared memory) took the 13.5 M
 // cells and 14 M points of a 512^3 threshold from 143 to 138 us, 655 MB at 4.7
-// TB/s.  (The words' data broadcast from shared memory in place of shuffles,
+// TB/s; batches of 8 words took that to 133.  (The words' data broadcast from shared memory in place of shuffles,
 // and four words at a time with their values a group ahead, took a fifth off
 // the instructions and no time.)
 __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restrict__ f,
@@ -243,16 +248,24 @@ __global__ void __launch_bounds__(256) k_thr_emit(Grid g, const float* __restric
   const int lane = threadIdx.x & 31;
   const uint32_t below = (1u << lane) - 1u;
   const bool conn32 = (reinterpret_cast<uintptr_t>(conn) & 31) == 0;
-  const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const unsigned wr = (unsigned)g.wr;
-  __shared__ float s_field[8][32][32];  // per warp: field value of bit `lane` of batch word s
+  __shared__ float s_field[8][kThrBatch][32];  // per warp: field value of bit `lane` of batch word s
   float (*const sf)[32] = s_field[threadIdx.x >> 5];
   __shared__ float s_coord[8][2][96];  // per warp, alternating words: the word's coordinates
-  for (long long a0 = warp0 * 32; a0 < A; a0 += nwarps * 32) {
+  // the block's batches of words are every gridDim.x-th one; its warps take
+  // them from a counter in shared memory (words differ widely in cost)
+  __shared__ unsigned s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  while (true) {
+    unsigned n = 0;
+    if (lane == 0) n = atomicAdd(&s_next, 1u);
+    const long long a0 =
+        ((long long)__shfl_sync(kFull, n, 0) * gridDim.x + blockIdx.x) * kThrBatch;
+    if (a0 >= A) break;
     // lane L gathers active word a0 + L
     ThrWord d{};
-    const int cnt = (int)min(32ll, A - a0);
+    const int cnt = (int)min((long long)kThrBatch, A - a0);
     if (lane < cnt) {
       d.w = __ldg(act + a0 + lane);
       d.u = __ldg(used + d.w);
@@ -400,9 +413,9 @@ void launch_thr_emit(const Grid& g, const float* f, const WordOffsets& o, const 
                      const uint32_t* used, Info* info, int32_t* conn, long long kcap,
                      float* coords, float* fout, long long ucap, int num_sms, cudaStream_t s) {
   // the active count lives on the device: one resident wave, grid-stride
-  const long long want = (g.R * g.wr + 255) / 256;
+  const long long want = (g.R * g.wr + 8 * kThrBatch - 1) / (8 * kThrBatch);
   const int blocks = resident_blocks(k_thr_emit, 256, 0, num_sms, want);
-  // an ordinary launch: the warps split the active words statically, so all
+  // an ordinary launch: the blocks split the active words statically, so all
   // blocks should start together on an idle device (launched early into the
   // SMs the scan frees, they measured 20 us slower at 512^3)
   k_thr_emit<<<blocks, 256, 0, s>>>(g, f, kept, used, o.wt, o.wv, o.act, info, conn, kcap, coords,
