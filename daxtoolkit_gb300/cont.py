@@ -36,8 +36,10 @@ def _ptr(t):
 
 
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    # the raw handle: building torch's Stream object took 3 of the 54 us of a call on a small grid
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _require_field(field, grid):

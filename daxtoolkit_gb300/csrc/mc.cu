@@ -191,7 +191,7 @@ __device__ __forceinline__ void list_words(const Grid& g, const uint32_t* __rest
 // wholly inside or outside, and the others are listed in shared memory.  Then
 // lane = listed word: its counts by word_tris.  (Counting in the first step
 // held every warp for its few words with a surface: 32 us for the 4.2 M words
-// of 512^3, now 25; a tile of the 201^3 Mandelbulb, nearly all of whose words
+// of 512^3, now 23; a tile of the 201^3 Mandelbulb, nearly all of whose words
 // have one, 133 us, now 15.)  The block writes the tile's counts with
 // whole-line stores and its totals (triangles, crossing edges, active words)
 // to tile_tot[0 / 1 / 2][tile] for the scan.
@@ -199,13 +199,16 @@ __device__ __forceinline__ void list_words(const Grid& g, const uint32_t* __rest
 // A set's tile with up to kCountSegments grids takes them one after another;
 // with more, each lane takes a word from its own grid: short ranges would
 // leave most of the block idle at each.
-template <bool SET>
-__global__ void __launch_bounds__(kCountThreads, 2) k_mc_count(GridSet S,
-                                                               const uint32_t* __restrict__ bits,
-                                                               uint32_t* __restrict__ wc,
-                                                               uint32_t* __restrict__ tile_tot,
-                                                               int tiles, int tile_begin,
-                                                               int tile_end) {
+//
+// BLOCKS an SM: a tile is faster with the registers of two, but where one grid
+// has more tiles than two an SM, three finish them sooner (from the
+// classification's end to the scan's, two and three: 38.6 and 34.7 us at 512^3,
+// 22.6 and 19.2 on a slice of 383 x 405 x 331, 393 tiles; 13.1 and 17.3 at 301
+// x 257 x 199, 125 tiles; 26.8 and 29.2 for a set of 32 grids, 352 tiles).
+template <bool SET, int BLOCKS>
+__global__ void __launch_bounds__(kCountThreads, BLOCKS)
+    k_mc_count(GridSet S, const uint32_t* __restrict__ bits, uint32_t* __restrict__ wc,
+               uint32_t* __restrict__ tile_tot, int tiles, int tile_begin, int tile_end) {
   constexpr int kWarps = kCountThreads / 32;
   __shared__ __align__(16) uint32_t s_wc[kScanTile];
   __shared__ unsigned short s_list[kScanTile];
@@ -471,10 +474,14 @@ void launch_word_scan(long long rowwords, const uint32_t* wc, const uint32_t* ti
              act, info, 0, SlabBounds{}, (uint32_t*)nullptr, abort);
 }
 
+static auto count_kernel(int tiles, int num_sms) {
+  return tiles > 2 * num_sms ? k_mc_count<false, 3> : k_mc_count<false, 2>;
+}
+
 void launch_mc_scan(const GridSet& S, const uint32_t* bits, const WordOffsets& o, Info* info,
                     int num_sms, cudaStream_t s) {
   const int tiles = word_scan_tiles(S.rowwords);
-  const auto kernel = S.count > 1 ? k_mc_count<true> : k_mc_count<false>;
+  const auto kernel = S.count > 1 ? k_mc_count<true, 2> : count_kernel(tiles, num_sms);
   // a block a tile, unless other frames are to find room on the SMs
   const int b1 = tuned_blocks_per_sm(kPassCount) > 0
                      ? resident_blocks(kernel, kCountThreads, 0, num_sms, tiles, kPassCount)
@@ -491,8 +498,9 @@ void launch_mc_scan_slab(const GridSet& S, const uint32_t* bits, const WordOffse
                          int pass, int num_sms, cudaStream_t s, cudaEvent_t after_count) {
   const int tiles = word_scan_tiles(S.rowwords);
   const int n = tile_end - tile_begin;
-  const int b1 = resident_blocks(k_mc_count<false>, kCountThreads, 0, num_sms, n, pass);
-  k_mc_count<false><<<b1, kCountThreads, 0, s>>>(S, bits, o.wc, o.tile, tiles, tile_begin, tile_end);
+  const auto kernel = count_kernel(n, num_sms);
+  const int b1 = resident_blocks(kernel, kCountThreads, 0, num_sms, n, pass);
+  kernel<<<b1, kCountThreads, 0, s>>>(S, bits, o.wc, o.tile, tiles, tile_begin, tile_end);
   if (after_count) cudaEventRecord(after_count, s);
   k_word_scan<true><<<n, 256, 0, s>>>(S.rowwords, o.wc, o.tile, tiles, o.wt, o.wv, o.act, info,
                                       tile_begin, B, slab_act, nullptr);
