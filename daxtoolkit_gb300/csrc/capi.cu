@@ -570,9 +570,8 @@ int dax_gb300_slice_count(const dax_gb300_uniform_grid* grid, const float* origi
   const daxgb::WordOffsets wo = L.offsets(d_scratch);
   // the row splits live in the active-word list (R <= R * wr entries), which
   // the scan rewrites afterwards
-  cudaMemsetAsync(at<Info>(d_scratch, L.info), 0, sizeof(Info), s);  // the error words
   daxgb::launch_slice_bits(g, S.one.plane_o, S.one.plane_n, iso, bits, daxgb::bit_words(g.P),
-                           wo.act, sms, s);
+                           wo.act, at<Info>(d_scratch, L.info), sms, s);
   if ((st = check_launch("slice classify kernels"))) return st;
   daxgb::launch_mc_scan(S, bits, wo, at<Info>(d_scratch, L.info), sms, s);
   return check_launch("count/scan kernels");

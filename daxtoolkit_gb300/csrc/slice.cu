@@ -22,6 +22,16 @@
 
 namespace daxgb {
 
+// The error word and the emit counters, cleared by the first kernel of a count
+// pass.
+__device__ __forceinline__ void clear_info(Info* info) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    info->error = 0;
+    info->ticket = 0;
+    info->done = 0;
+  }
+}
+
 // Per-point classification, for planes and grids whose values may overflow
 // or be NaN.  Each warp walks a contiguous run of steps, one 32-bit word of
 // the flat bit stream (bit p of word p / 32) per step; lane l holds point
@@ -34,8 +44,9 @@ namespace daxgb {
 __global__ void __launch_bounds__(256) k_slice_points(Grid g, float3 o, float3 n, float iso,
                                                       long long steps, long long per,
                                                       unsigned long long mnx,
-                                                      uint32_t* __restrict__ bits) {
+                                                      uint32_t* __restrict__ bits, Info* init) {
   extern __shared__ float s_tx[];  // [nx]: n.x * (x(i) - o.x)
+  clear_info(init);
   for (int i = threadIdx.x; i < g.nx; i += blockDim.x)
     s_tx[i] = __fmul_rn(n.x, __fsub_rn(coord(g.ox, g.sx, i, g.mx), o.x));
   __syncthreads();
@@ -131,7 +142,9 @@ __device__ __forceinline__ bool slice_inside(const Grid& g, float3 o, float3 n, 
 // split[r] = number of leading points of row r whose test equals point 0's;
 // bit 31 holds point 0's test.
 __global__ void __launch_bounds__(256) k_slice_rows(Grid g, float3 o, float3 n, float iso,
-                                                    uint32_t* __restrict__ split) {
+                                                    uint32_t* __restrict__ split, Info* init) {
+  pdl_trigger();
+  clear_info(init);
   for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < g.R;
        r += (long long)gridDim.x * blockDim.x) {
     int j, k;
@@ -154,6 +167,8 @@ __global__ void __launch_bounds__(256) k_slice_words(Grid g, unsigned long long 
                                                      const uint32_t* __restrict__ split,
                                                      uint32_t* __restrict__ bits,
                                                      long long nwords) {
+  pdl_trigger();
+  pdl_wait();  // the rows' splits
   for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < nwords;
        w += (long long)gridDim.x * blockDim.x) {
     const long long p0 = w << 5;
@@ -226,12 +241,14 @@ bool slice_rows_exact(const Grid& g, float3 o, float3 n) {
 }
 
 void launch_slice_bits(const Grid& g, float3 o, float3 n, float iso, uint32_t* bits,
-                       long long nwords, uint32_t* row_scratch, int num_sms, cudaStream_t s) {
+                       long long nwords, uint32_t* row_scratch, Info* init, int num_sms,
+                       cudaStream_t s) {
   if (row_scratch && std::isfinite(iso) && slice_rows_exact(g, o, n)) {
     const int rb = resident_blocks(k_slice_rows, 256, 0, num_sms, (g.R + 255) / 256);
-    k_slice_rows<<<rb, 256, 0, s>>>(g, o, n, iso, row_scratch);
+    k_slice_rows<<<rb, 256, 0, s>>>(g, o, n, iso, row_scratch, init);
     const int wb = resident_blocks(k_slice_words, 256, 0, num_sms, (nwords + 255) / 256);
-    k_slice_words<<<wb, 256, 0, s>>>(g, div_multiplier((unsigned)g.nx), row_scratch, bits, nwords);
+    launch_pdl(k_slice_words, (unsigned)wb, 256u, 0, s, g, div_multiplier((unsigned)g.nx), row_scratch,
+               bits, nwords);
     return;
   }
   const size_t smem = tx_smem(k_slice_points, g);
@@ -242,7 +259,7 @@ void launch_slice_bits(const Grid& g, float3 o, float3 n, float iso, uint32_t* b
   long long per = (nwords + warps - 1) / warps;
   per = (per + 31) / 32 * 32;
   k_slice_points<<<blocks, 256, smem, s>>>(g, o, n, iso, nwords, per,
-                                           div_multiplier((unsigned)g.nx), bits);
+                                           div_multiplier((unsigned)g.nx), bits, init);
 }
 
 void launch_slice_field(const Grid& g, float3 o, float3 n, float* out, int num_sms,
