@@ -209,8 +209,8 @@ __device__ __forceinline__ void grad_adjoint_task(const Grid& g, const float* __
 
 __host__ __device__ inline int adj_nxw(const Grid& g) { return (g.nx + kMarchCols - 1) / kMarchCols; }
 __host__ __device__ inline int adj_bands(const Grid& g) { return (g.ny + kAdjBand - 1) / kAdjBand; }
-__host__ __device__ inline MarchTiles adj_set_tiles(const Grid& g) {
-  return march_tiles(adj_nxw(g), adj_bands(g), g.nz, (g.nz + kSeg - 1) / kSeg);
+__host__ __device__ inline MarchTiles adj_set_tiles(const Grid& g, int seg) {
+  return march_tiles(adj_nxw(g), adj_bands(g), g.nz, (g.nz + seg - 1) / seg);
 }
 
 __global__ void __launch_bounds__(32, kAdjMinBlocks)
@@ -221,11 +221,11 @@ __global__ void __launch_bounds__(32, kAdjMinBlocks)
 // A grid set: the block's grid (block0 as in k_cell_gradient_set); cell
 // gradients and the output field are concatenated over the set.
 __global__ void __launch_bounds__(32, kAdjMinBlocks)
-    k_grad_adjoint_set(GridSet S, const long long* __restrict__ block0,
+    k_grad_adjoint_set(GridSet S, const long long* __restrict__ block0, int seg,
                        const float* __restrict__ dg, float* __restrict__ out) {
   const int si = block_slot(block0, S.count, blockIdx.x);
   const Grid g = S.slots[si].g;
-  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0, adj_set_tiles(g),
+  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0, adj_set_tiles(g, seg),
                     (long long)blockIdx.x - __ldg(block0 + si));
 }
 
@@ -432,50 +432,54 @@ __global__ void __launch_bounds__(256) k_edge_adjoint(Grid g, const float* __res
     edge_adjoint_words(g, f, iso, bits, wv, dverts, out, w0);
 }
 
-// A grid set: each block takes 256 consecutive row words of its grid
+// A grid set: each block takes `words` consecutive row words of its grid
 // (block0 per grid); bits, word offsets and vertex gradients are the set's,
 // the output field is concatenated over the set.
-__global__ void __launch_bounds__(256) k_edge_adjoint_set(GridSet S,
-                                                          const long long* __restrict__ block0,
-                                                          const uint32_t* __restrict__ bits,
-                                                          const uint32_t* __restrict__ wv,
-                                                          const float* __restrict__ dverts,
-                                                          float* __restrict__ out) {
+__global__ void __launch_bounds__(256, 4)
+    k_edge_adjoint_set(GridSet S, const long long* __restrict__ block0, int words,
+                       const uint32_t* __restrict__ bits, const uint32_t* __restrict__ wv,
+                       const float* __restrict__ dverts, float* __restrict__ out) {
   const int si = block_slot(block0, S.count, blockIdx.x);
   const GridSlot& sl = S.slots[si];
   const Grid g = sl.g;
-  const long long w0 = ((long long)blockIdx.x - __ldg(block0 + si)) * 256 + (threadIdx.x & ~31);
-  if (w0 < g.R * g.wr)
+  const long long first = ((long long)blockIdx.x - __ldg(block0 + si)) * words;
+  const long long end = min(first + words, g.R * g.wr);
+#pragma unroll 1
+  for (long long w0 = first + (threadIdx.x & ~31); w0 < end; w0 += 256)
     edge_adjoint_words(g, sl.field, sl.iso, bits + sl.word0, wv + sl.rw0, dverts,
                        out + sl.point0, w0);
 }
 
-long long adjoint_grad_blocks(const Grid& g) {
-  return adj_set_tiles(g).tasks;
+MarchBox adjoint_box(const Grid& g) { return {(long long)adj_nxw(g) * adj_bands(g), g.nz}; }
+int adjoint_wave(int num_sms) {
+  return resident_blocks(k_grad_adjoint_set, 32, kAdjSmem, num_sms, 1ll << 30);
 }
-long long adjoint_edge_blocks(const Grid& g) { return (g.R * g.wr + 255) / 256; }
+long long adjoint_grad_blocks(const Grid& g, int seg) {
+  return adj_set_tiles(g, seg).tasks;
+}
+long long adjoint_edge_blocks(const Grid& g, int words) { return (g.R * g.wr + words - 1) / words; }
 
 void launch_field_adjoint_set(const GridSet& S, const long long* grad_block0,
-                              long long grad_blocks, const long long* edge_block0,
-                              long long edge_blocks, long long points, const uint32_t* bits,
+                              long long grad_blocks, int seg, const long long* edge_block0,
+                              long long edge_blocks, int edge_words, long long points,
+                              const uint32_t* bits,
                               const uint32_t* wv, const float* dverts, const float* dgrad,
                               float* out, cudaStream_t s) {
   if (dgrad && grad_blocks > 0)
-    k_grad_adjoint_set<<<(unsigned)grad_blocks, 32, kAdjSmem, s>>>(S, grad_block0, dgrad,
+    k_grad_adjoint_set<<<(unsigned)grad_blocks, 32, kAdjSmem, s>>>(S, grad_block0, seg, dgrad,
                                                                                out);
   else
     cudaMemsetAsync(out, 0, (size_t)points * sizeof(float), s);
   if (dverts && edge_blocks > 0)
-    k_edge_adjoint_set<<<(unsigned)edge_blocks, 256, 0, s>>>(S, edge_block0, bits, wv, dverts,
-                                                             out);
+    k_edge_adjoint_set<<<(unsigned)edge_blocks, 256, 0, s>>>(S, edge_block0, edge_words, bits, wv,
+                                                             dverts, out);
 }
 
 void launch_field_adjoint(const Grid& g, const float* f, float iso, const uint32_t* bits,
                           const WordOffsets* o, const float* dverts, const float* dgrad,
                           float* out, int num_sms, cudaStream_t s) {
   if (dgrad) {
-    const int wave = resident_blocks(k_grad_adjoint, 32, kAdjSmem, num_sms, 1ll << 30);
-    const MarchTiles mt = march_tiles_for(adj_nxw(g), adj_bands(g), g.nz, wave);
+    const MarchTiles mt = march_tiles_for(adj_nxw(g), adj_bands(g), g.nz, adjoint_wave(num_sms));
     k_grad_adjoint<<<(unsigned)mt.tasks, 32, kAdjSmem, s>>>(g, dgrad, out, mt);
   } else {
     cudaMemsetAsync(out, 0, (size_t)g.P * sizeof(float), s);

@@ -324,6 +324,8 @@ struct dax_gb300_mc_batch {
   long long cells = 0, points = 0;
   long long* d_blk = nullptr;
   long long blk_total[3] = {0, 0, 0};
+  int grad_seg = 1, adj_seg = 1;  // planes a segment of the set's tiles
+  int edge_words = 256;           // row words a block of the vertex adjoint
   bool grad_vec = true, grad_loadv = true;
 
   daxgb::GridSet set() const {
@@ -1161,10 +1163,22 @@ int dax_gb300_mc_batch_create(int num_grids, const dax_gb300_uniform_grid* grids
   b->L = mc_layout_words(b->rowwords, b->words, b->off_goff + 16 * (size_t)(num_grids + 1));
   // per grid, the first block of each grid-set launch
   std::vector<long long> blk(3 * (size_t)(num_grids + 1), 0);
+  std::vector<daxgb::MarchBox> gbox(num_grids), abox(num_grids);
+  long long large = 0;
   for (int i = 0; i < num_grids; ++i) {
     const Grid& g = b->slots[i].g;
-    const long long n[3] = {daxgb::grad_blocks(g), daxgb::adjoint_grad_blocks(g),
-                            daxgb::adjoint_edge_blocks(g)};
+    gbox[i] = daxgb::grad_box(g);
+    abox[i] = daxgb::adjoint_box(g);
+    large += daxgb::adjoint_edge_blocks(g, daxgb::kEdgeWordsMost);
+  }
+  b->grad_seg = daxgb::march_seg(gbox.data(), num_grids, daxgb::grad_wave(num_sms()), daxgb::kGradSeg);
+  b->adj_seg = daxgb::march_seg(abox.data(), num_grids, daxgb::adjoint_wave(num_sms()), daxgb::kSeg);
+  // two waves of the larger blocks, four an SM, or more
+  b->edge_words = large >= 8ll * num_sms() ? daxgb::kEdgeWordsMost : daxgb::kEdgeWordsLeast;
+  for (int i = 0; i < num_grids; ++i) {
+    const Grid& g = b->slots[i].g;
+    const long long n[3] = {daxgb::grad_blocks(g, b->grad_seg), daxgb::adjoint_grad_blocks(g, b->adj_seg),
+                            daxgb::adjoint_edge_blocks(g, b->edge_words)};
     for (int k = 0; k < 3; ++k) blk[k * (num_grids + 1) + i + 1] = blk[k * (num_grids + 1) + i] + n[k];
   }
   for (int k = 0; k < 3; ++k) b->blk_total[k] = blk[k * (num_grids + 1) + num_grids];
@@ -1260,7 +1274,7 @@ int dax_gb300_mc_batch_sizes(const dax_gb300_mc_batch* b, int64_t* num_cells,
 int dax_gb300_mc_batch_cell_gradient(const dax_gb300_mc_batch* b, float* d_out, void* stream) {
   if (!b || (!d_out && b->cells > 0)) return fail(DAX_GB300_ERROR_BAD_VALUE, "NULL batch or output");
   const bool vec = b->grad_vec && (reinterpret_cast<uintptr_t>(d_out) & 7) == 0;
-  daxgb::launch_cell_gradient_set(b->set_for_sets(), b->d_blk, b->blk_total[0], vec, b->grad_loadv,
+  daxgb::launch_cell_gradient_set(b->set_for_sets(), b->d_blk, b->blk_total[0], b->grad_seg, vec, b->grad_loadv,
                                   d_out, static_cast<cudaStream_t>(stream));
   return check_launch("batch cell gradient kernel");
 }
@@ -1276,7 +1290,8 @@ int dax_gb300_mc_batch_field_adjoint(const dax_gb300_mc_batch* b, const void* d_
   void* sc = const_cast<void*>(d_scratch);
   const daxgb::WordOffsets wo = d_scratch ? b->L.offsets(sc) : daxgb::WordOffsets{};
   daxgb::launch_field_adjoint_set(b->set_for_sets(), b->d_blk + n, b->blk_total[1],
-                                  b->d_blk + 2 * n, b->blk_total[2], b->points,
+                                  b->adj_seg, b->d_blk + 2 * n, b->blk_total[2], b->edge_words,
+                                  b->points,
                                   d_scratch ? at<uint32_t>(sc, b->L.bits) : nullptr, wo.wv,
                                   d_grad_vertices, d_grad_cell_gradients, d_grad_fields,
                                   static_cast<cudaStream_t>(stream));

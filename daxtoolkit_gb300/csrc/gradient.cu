@@ -8,7 +8,7 @@
 //
 // A warp marches along z over a tile of kGradCols = 62 cells in x (two per
 // lane on lanes 0..30; lane 31 loads the tile's last two point columns and
-// owns no cell), kGradBand cell rows in y and kGradSeg cell planes.  Each
+// owns no cell), kGradBand cell rows in y and a segment of cell planes.  Each
 // lane copies its two point columns of every point plane of the tile
 // (kGradBand + 1 rows; one 8-byte copy per row where the rows allow it)
 // into the warp's ring in shared memory with cp.async, kGradDepth planes
@@ -239,7 +239,7 @@ __device__ __forceinline__ void cell_gradient_task(const Grid& g, const float* _
   const int i = kGradCols * xw + 2 * lane;  // the lane's first point (and cell) column
   const bool c0 = i < g.nx, c1 = i + 1 < g.nx;
   const int j0 = band * kGradBand;
-  const int k0 = seg * kGradSeg, k1 = min(k0 + kGradSeg, cz);
+  const int k0 = seg * mt.seg, k1 = min(k0 + mt.seg, cz);
 
   GradTile T;
   T.rows = min(kGradBand, cy - j0);
@@ -312,58 +312,57 @@ __global__ void __launch_bounds__(kGradWarps * 32, kGradMinBlocks)
                                  (long long)blockIdx.x * kGradWarps + (threadIdx.x >> 5));
 }
 
-// Cell tiles of one grid's CellGradient.
-__host__ __device__ inline MarchTiles grad_tiles(const Grid& g) {
-  MarchTiles mt;
-  mt.nxw = (g.nx - 1 + kGradCols - 1) / kGradCols;
-  mt.nband = (g.ny - 1 + kGradBand - 1) / kGradBand;
-  mt.nseg = (g.nz - 1 + kGradSeg - 1) / kGradSeg;
-  mt.tasks = (long long)mt.nxw * mt.nband * mt.nseg;
-  return mt;
+__host__ __device__ inline int grad_nxw(const Grid& g) { return (g.nx - 1 + kGradCols - 1) / kGradCols; }
+__host__ __device__ inline int grad_bands(const Grid& g) { return (g.ny - 1 + kGradBand - 1) / kGradBand; }
+__host__ __device__ inline MarchTiles grad_tiles(const Grid& g, int seg) {
+  return march_tiles(grad_nxw(g), grad_bands(g), g.nz - 1, (g.nz - 1 + seg - 1) / seg);
 }
 
 // A grid set: block b works for the grid whose first block (block0) is the
 // last at or before b; the grid's gradients start at its first cell.
 template <bool VEC, bool LOADV>
 __global__ void __launch_bounds__(kGradWarps * 32, kGradMinBlocks)
-    k_cell_gradient_set(GridSet S, const long long* __restrict__ block0,
+    k_cell_gradient_set(GridSet S, const long long* __restrict__ block0, int seg,
                         float* __restrict__ out) {
   const int si = block_slot(block0, S.count, blockIdx.x);
   const Grid g = S.slots[si].g;
-  cell_gradient_task<VEC, LOADV>(g, S.slots[si].field, out + 3 * S.slots[si].cell0, grad_tiles(g),
+  cell_gradient_task<VEC, LOADV>(g, S.slots[si].field, out + 3 * S.slots[si].cell0, grad_tiles(g, seg),
                                  ((long long)blockIdx.x - __ldg(block0 + si)) * kGradWarps +
                                      (threadIdx.x >> 5));
 }
 
-long long grad_blocks(const Grid& g) {
+MarchBox grad_box(const Grid& g) {
+  if (g.nx < 2 || g.ny < 2 || g.nz < 2) return {0, 0};
+  return {(long long)grad_nxw(g) * grad_bands(g), g.nz - 1};
+}
+int grad_wave(int num_sms) {
+  return kGradWarps *
+         resident_blocks(k_cell_gradient<true, false>, kGradWarps * 32, 0, num_sms, 1ll << 30);
+}
+long long grad_blocks(const Grid& g, int seg) {
   if (g.nx < 2 || g.ny < 2 || g.nz < 2) return 0;
-  return (grad_tiles(g).tasks + kGradWarps - 1) / kGradWarps;
+  return (grad_tiles(g, seg).tasks + kGradWarps - 1) / kGradWarps;
 }
 
 void launch_cell_gradient_set(const GridSet& S, const long long* block0, long long blocks,
-                              bool vec, bool loadv, float* out, cudaStream_t s) {
+                              int seg, bool vec, bool loadv, float* out, cudaStream_t s) {
   if (blocks <= 0) return;
   const dim3 block(kGradWarps * 32);
   const unsigned nb = (unsigned)blocks;
   if (vec && loadv)
-    k_cell_gradient_set<true, true><<<nb, block, 0, s>>>(S, block0, out);
+    k_cell_gradient_set<true, true><<<nb, block, 0, s>>>(S, block0, seg, out);
   else if (vec)
-    k_cell_gradient_set<true, false><<<nb, block, 0, s>>>(S, block0, out);
+    k_cell_gradient_set<true, false><<<nb, block, 0, s>>>(S, block0, seg, out);
   else if (loadv)
-    k_cell_gradient_set<false, true><<<nb, block, 0, s>>>(S, block0, out);
+    k_cell_gradient_set<false, true><<<nb, block, 0, s>>>(S, block0, seg, out);
   else
-    k_cell_gradient_set<false, false><<<nb, block, 0, s>>>(S, block0, out);
+    k_cell_gradient_set<false, false><<<nb, block, 0, s>>>(S, block0, seg, out);
 }
 
 void launch_cell_gradient(const Grid& g, const float* f, float* out, int num_sms, cudaStream_t s) {
-  (void)num_sms;
-  const int cx = g.nx - 1, cy = g.ny - 1, cz = g.nz - 1;
-  if (cx < 1 || cy < 1 || cz < 1) return;
-  MarchTiles mt;  // cell tiles
-  mt.nxw = (cx + kGradCols - 1) / kGradCols;
-  mt.nband = (cy + kGradBand - 1) / kGradBand;
-  mt.nseg = (cz + kGradSeg - 1) / kGradSeg;
-  mt.tasks = (long long)mt.nxw * mt.nband * mt.nseg;
+  const MarchBox box = grad_box(g);
+  if (box.planes < 1) return;
+  const MarchTiles mt = grad_tiles(g, march_seg(&box, 1, grad_wave(num_sms), kGradSeg));
   const unsigned blocks = (unsigned)((mt.tasks + kGradWarps - 1) / kGradWarps);
   const dim3 block(kGradWarps * 32);
   const bool vec = (reinterpret_cast<uintptr_t>(out) & 7) == 0;

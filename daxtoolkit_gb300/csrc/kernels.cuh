@@ -250,13 +250,17 @@ void launch_thr_emit(const Grid& g, const float* f, const WordOffsets& o, const 
 // marched along z; an adjoint block is one warp.  Band heights and register
 // budgets (blocks per SM) were chosen by timing on GB300.
 constexpr int kMarchCols = 31;
-constexpr int kSeg = 32;            // planes a segment of a grid set's tiles, about
+constexpr int kSeg = 32;            // planes a segment of a grid set's adjoint tiles, at most
 constexpr int kGradBand = 4;        // cell rows per CellGradient tile
-constexpr int kGradSeg = 16;        // cell planes per CellGradient tile
+constexpr int kGradSeg = 16;        // cell planes per CellGradient tile, at most
 constexpr int kGradWarps = 4;       // CellGradient tiles (warps) per block
 constexpr int kGradMinBlocks = 4;
 constexpr int kAdjBand = 8;         // point rows per adjoint tile
 constexpr int kAdjMinBlocks = 28;
+// Row words a block of a grid set's vertex adjoint: a block spends much of its
+// time finding its grid, so large sets take the larger count (72 -> 54 us for
+// 32 grids of 45 M points, with four blocks an SM instead of three).
+constexpr int kEdgeWordsMost = 512, kEdgeWordsLeast = 256;
 
 struct MarchTiles {
   int nxw, nband, nseg;  // tiles along x, y, z
@@ -272,6 +276,26 @@ __host__ __device__ inline MarchTiles march_tiles(int nxw, int nband, int planes
   mt.tasks = (long long)nxw * nband * mt.nseg;
   return mt;
 }
+constexpr int kLeastSeg = 4;  // planes a segment at least: its first plane is read for nothing
+
+// The planes a segment of grids too small to fill a wave of `wave` tiles with
+// segments of `most` planes: the fewest with which all tiles still run at once
+// (a tile takes its planes one after another, about 1 us each: the adjoint of 6
+// grids of 32^3 to 80^3 took 39 us with segments of 32, now 11; of one grid of
+// 100 x 90 x 80 40 us, now 8).
+struct MarchBox {
+  long long columns;  // tiles in x and y
+  int planes;
+};
+inline int march_seg(const MarchBox* box, int count, long long wave, int most) {
+  for (int seg = kLeastSeg; seg < most; ++seg) {
+    long long n = 0;
+    for (int i = 0; i < count; ++i) n += box[i].columns * ((box[i].planes + seg - 1) / seg);
+    if (n <= wave) return seg;
+  }
+  return most;
+}
+
 // The number of segments that wastes least of one grid's adjoint: a wave of
 // `wave` resident tiles runs as long as a segment, which also reads one halo
 // plane and takes about a plane's time to start.  (Cutting the planes of all
@@ -281,7 +305,7 @@ __host__ __device__ inline MarchTiles march_tiles(int nxw, int nband, int planes
 inline MarchTiles march_tiles_for(int nxw, int nband, int planes, long long wave) {
   MarchTiles best{};
   long long least = -1;
-  for (int nseg = (planes + 63) / 64; nseg <= (planes + 11) / 12; ++nseg) {
+  for (int nseg = (planes + 63) / 64; nseg <= (planes + kLeastSeg - 1) / kLeastSeg; ++nseg) {
     const MarchTiles mt = march_tiles(nxw, nband, planes, nseg);
     const long long cost = (mt.tasks + wave - 1) / wave * (mt.seg + 2);
     if (least < 0 || cost < least) {
@@ -303,19 +327,24 @@ void launch_cell_gradient(const Grid& g, const float* f, float* out, int num_sms
 // Grid sets (one launch for all grids; block0[slot] = the grid's first block,
 // from the per-grid block counts below; per-cell and per-point arrays are
 // concatenated over the set at the slots' cell0 / point0).
-long long grad_blocks(const Grid& g);
-long long adjoint_grad_blocks(const Grid& g);
-long long adjoint_edge_blocks(const Grid& g);
+MarchBox grad_box(const Grid& g);
+MarchBox adjoint_box(const Grid& g);
+int grad_wave(int num_sms);     // resident CellGradient tiles
+int adjoint_wave(int num_sms);  // resident adjoint tiles
+long long grad_blocks(const Grid& g, int seg);
+long long adjoint_grad_blocks(const Grid& g, int seg);
+long long adjoint_edge_blocks(const Grid& g, int words);
 // vec: every grid's output 8-byte aligned; loadv: every grid's nx even and
 // field 8-byte aligned (the single-grid kernel's fast paths).
 void launch_cell_gradient_set(const GridSet& S, const long long* block0, long long blocks,
-                              bool vec, bool loadv, float* out, cudaStream_t s);
+                              int seg, bool vec, bool loadv, float* out, cudaStream_t s);
 // dL/dfield of every grid, out[points]: the gradient term from dgrad (or
 // zero) then the vertex term from dverts (the set's merged vertices; needs
 // the set's count pass: bits and word offsets wv).
 void launch_field_adjoint_set(const GridSet& S, const long long* grad_block0,
-                              long long grad_blocks, const long long* edge_block0,
-                              long long edge_blocks, long long points, const uint32_t* bits,
+                              long long grad_blocks, int seg, const long long* edge_block0,
+                              long long edge_blocks, int edge_words, long long points,
+                              const uint32_t* bits,
                               const uint32_t* wv, const float* dverts, const float* dgrad,
                               float* out, cudaStream_t s);
 
