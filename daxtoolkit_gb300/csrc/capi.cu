@@ -268,7 +268,7 @@ int count_pass(int mode, const dax_gb300_uniform_grid* grid, const float* field,
   daxgb::launch_thr_count(g, bits, at<uint32_t>(scratch, L.kept), at<uint32_t>(scratch, L.used),
                           o.wc, o.tile, sms, s);
   daxgb::launch_word_scan(g.R * g.wr, o.wc, o.tile, o.wt, o.wv, o.act, at<Info>(scratch, L.m.info),
-                          s);
+                          true, s);
   return check_launch("threshold count/scan kernels");
 }
 

@@ -778,7 +778,7 @@ int launch_fused_count(int mode, const Grid& g, const float* f, float a, float b
   if (e != cudaSuccess) return (int)e;
   // the per-word offsets, the active-word list and the totals (the abort word
   // becomes kErrTimeout)
-  launch_word_scan(A.W, o.wc, o.tile, o.wt, o.wv, o.act, info, s, fctl + 1);
+  launch_word_scan(A.W, o.wc, o.tile, o.wt, o.wv, o.act, info, true, s, fctl + 1);
   return (int)cudaGetLastError();
 }
 

@@ -108,7 +108,8 @@ inline int resident_blocks(K kernel, int threads, size_t smem, int num_sms, long
 // per tile of kScanTile words, the totals of a, of b and of non-zero words
 // (tile[0 / 1 / 2][tiles]); launch_word_scan turns them into per-word
 // exclusive offsets wt (a), wv (b) (uint32[rowwords + 1]; entry rowwords
-// holds the totals), the compacted list act of the non-zero words, and the
+// holds the totals; sparse: those of non-zero words and of the words before
+// them, the first and entry rowwords only), the compacted list act of the non-zero words, and the
 // totals and error word in Info.
 constexpr int kScanItems = 16;               // words per thread in a tile
 constexpr int kScanTile = 256 * kScanItems;  // words per tile
@@ -184,8 +185,8 @@ int fused_unit_stages();
 // abort (optional): a word that, when non-zero, makes the scan report
 // kErrTimeout (the fused count pass's abort word).
 void launch_word_scan(long long rowwords, const uint32_t* wc, const uint32_t* tile_tot,
-                      uint32_t* wt, uint32_t* wv, uint32_t* act, Info* info, cudaStream_t s,
-                      const uint32_t* abort = nullptr);
+                      uint32_t* wt, uint32_t* wv, uint32_t* act, Info* info, bool sparse,
+                      cudaStream_t s, const uint32_t* abort = nullptr);
 // Marching cubes K2a (counts: triangles, crossing edges) + K2b.
 void launch_mc_scan(const GridSet& S, const uint32_t* bits, const WordOffsets& o, Info* info,
                     int num_sms, cudaStream_t s);

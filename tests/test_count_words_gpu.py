@@ -66,3 +66,21 @@ def test_unmerged_vertices_of_a_set():
     verts, conn = verts.cpu().numpy(), conn.cpu().numpy()
     for i, d in enumerate(sets):
         _check((verts[3 * tri[i]:3 * tri[i + 1]], conn[tri[i]:tri[i + 1]]), d, fields[i], 0.5, merge=False)
+
+
+@pytest.mark.parametrize("dims", [(300, 40, 30), (161, 61, 43), (8192, 3, 3)])
+def test_ids_across_words_without_edges(dims):
+    """Sparse surfaces: a plane across x puts the only edges of long stretches of rows next to a word's last cell, whose
+    far corners take their ids from the offset of a word that has none.  The scratch is dirtied by another surface."""
+    import torch
+    from daxtoolkit_gb300 import cont
+    nx, ny, nz = dims
+    grid, scratch = cont.UniformGrid(dims), cont.Scratch()
+    cont.marching_cubes(grid, torch.from_numpy(_field(dims, 7)).cuda(), 0.5, scratch=scratch)
+    x = np.arange(nx, dtype=np.float32)
+    for cut in (31, 32, 63, 127, 128, nx - 2):
+        f = np.broadcast_to(x + 0.003 * np.arange(ny, dtype=np.float32)[:, None], (nz, ny, nx)).astype(np.float32)
+        f[1:, ::3] += 0.75
+        f = np.ascontiguousarray(f.ravel())
+        out = cont.marching_cubes(grid, torch.from_numpy(f).cuda(), cut + 0.5, scratch=scratch)
+        _check((out["verts"].cpu().numpy(), out["conn"].cpu().numpy()), dims, f, cut + 0.5)
