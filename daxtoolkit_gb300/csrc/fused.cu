@@ -22,7 +22,7 @@
 //       tiles.  Blocks take tiles from the queue (one per unit while units
 //       are left, all that remain after) and count them from the bit stream
 //       in L2 -- the packed counts wc and per-tile totals of k_mc_count, or
-//       the kept / used masks, counts and totals of k_thr_kept + k_thr_used,
+//       the kept / used masks, counts and totals of k_thr_words,
 //       bit for bit.
 //
 // So the counts of plane k run while other blocks stream the planes after
@@ -382,8 +382,8 @@ __device__ __forceinline__ uint32_t kept_of(const Grid& g, const uint32_t* bits,
   return a & a1 & b & b1 & c & c1 & d & d1 & low_mask(g.nx - 1 - 32 * m);
 }
 
-// Threshold: kept and used masks of row words g0..g0+3 (as k_thr_kept and
-// k_thr_used: kept = cells whose 8 corners are in range, used = points that
+// Threshold: kept and used masks of row words g0..g0+3 (as k_thr_words:
+// kept = cells whose 8 corners are in range, used = points that
 // are a corner of a kept cell of cell rows (j-1..j, k-1..k)), written to the
 // kept / used arrays; packed counts popc(kept) << 16 | popc(used).
 __device__ __forceinline__ void thr_counts4(const FusedArgs& A, long long g0, uint32_t (&out)[4]) {

@@ -1,7 +1,7 @@
 // Cell threshold on the in-range bit stream (bit = lo <= f <= hi), on the
 // row-word pipeline marching cubes uses.
 //
-// K2a (k_thr_kept, k_thr_used): per row word w = (point row r = (j, k), word m)
+// K2a (k_thr_words): per row word w = (point row r = (j, k), word m)
 //     kept[w] = cells 32m .. 32m+31 of cell row r whose 8 corners are all in
 //               range (ThresholdFunction, dax/worklet/Threshold.h:30-66)
 //     used[w] = points 32m .. 32m+31 of point row r that are a corner of a
@@ -27,183 +27,124 @@
 
 namespace daxgb {
 
-// Bit positions fit in 32 bits: grids hold fewer than 2^31 points, and the
-// largest position read, a point plus two planes, stays below 2^32.
-__device__ __forceinline__ uint32_t bits_at_u32(const uint32_t* __restrict__ bits, uint32_t pos) {
-  return __funnelshift_r(__ldg(bits + (pos >> 5)), __ldg(bits + (pos >> 5) + 1), pos & 31u);
+// Pairs of a point row: bit x says whether points 32m + x and 32m + x + 1 are
+// both in range.
+__device__ __forceinline__ uint32_t row_pairs(const uint32_t* __restrict__ bits, unsigned pos) {
+  const uint32_t* const s = bits + (pos >> 5);
+  const uint32_t x0 = __ldg(s), x1 = __ldg(s + 1);
+  return __funnelshift_r(x0, x1, pos) & __funnelshift_rc(x0, x1, (pos & 31u) + 1u);
 }
 
-// Kept mask of cell-row word w (0 on rows without cells).
-__device__ __forceinline__ uint32_t kept_word(const Grid& g, const uint32_t* __restrict__ bits,
-                                              uint32_t w) {
-  const uint32_t nx = (uint32_t)g.nx, dy = nx, dz = nx * (uint32_t)g.ny;
-  int mi, ji, ki;
-  const uint32_t r = split_word(g, w, mi);
-  split_row(g, r, ji, ki);
-  const uint32_t m = (uint32_t)mi, j = (uint32_t)ji, k = (uint32_t)ki;
-  if (j + 1 >= (uint32_t)g.ny || k + 1 >= (uint32_t)g.nz) return 0u;
-  const uint32_t pos = r * nx + 32u * m;
-  const uint32_t p0 = pos, p1 = pos + dy, p2 = pos + dz, p3 = pos + dy + dz;
-  return bits_at_u32(bits, p0) & bits_at_u32(bits, p0 + 1) & bits_at_u32(bits, p1) &
-         bits_at_u32(bits, p1 + 1) & bits_at_u32(bits, p2) & bits_at_u32(bits, p2 + 1) &
-         bits_at_u32(bits, p3) & bits_at_u32(bits, p3 + 1) & low_mask(g.nx - 1 - 32 * (int)m);
+// The pairs of a point row that the row one plane down (x) and up (y) has too;
+// none across the grid's ends, nor for a row past its last.
+__device__ __forceinline__ uint2 plane_pairs(const uint32_t* __restrict__ bits, unsigned pos,
+                                             unsigned dz, int k, int nz) {
+  uint2 q = make_uint2(0u, 0u);
+  if (k < nz) {
+    const uint32_t b = row_pairs(bits, pos);
+    if (k > 0) q.x = b & row_pairs(bits, pos - dz);
+    if (k + 1 < nz) q.y = b & row_pairs(bits, pos + dz);
+  }
+  return q;
 }
 
-// K2a, first pass: kept masks of every cell-row word, four consecutive words
-// per thread; four words of one row come from five bit-word fetches per
-// corner row.
-__global__ void __launch_bounds__(256) k_thr_kept(Grid g, const uint32_t* __restrict__ bits,
-                                                  uint32_t* __restrict__ kept) {
+// K2a: one block per tile of kScanTile words (grid-stride over tiles).  A lane
+// walks down one word column over `depth` consecutive point rows: the pairs of
+// a row, in its plane and combined with the planes below and above, serve the
+// cells of the row and of the one before, and the kept cells between two rows
+// the used points of both.  Consecutive lanes take consecutive words; lane 0
+// repeats the word before lane 1's, whose last cell lane 1's first point may
+// belong to, and writes nothing.  A grid has fewer than 2^31 points, so bit
+// positions are 32-bit; rows are at most 8192 points, 256 words, long.  kept is
+// written where a point is used.  (Kept masks and used masks in two passes, four
+// words a lane: from the classification's end to the scan's 40 us at 512^3, 16
+// at 200 x 180 x 150, 17 at 60^3; now 34, 10 and 11, and with two blocks an SM
+// in place of four 39, 9 and 11.)
+constexpr int kThrThreads = 512;
+__global__ void __launch_bounds__(kThrThreads, 4)
+    k_thr_words(Grid g, const uint32_t* __restrict__ bits, uint32_t* __restrict__ kept,
+                uint32_t* __restrict__ used, uint32_t* __restrict__ wc,
+                uint32_t* __restrict__ tile_tot, int tiles) {
+  constexpr unsigned kWarps = kThrThreads / 32, kCols = 31;
+  __shared__ uint32_t s_sum[3];  // the tile's kept cells, used points and active words
   pdl_trigger();
   pdl_wait();  // the classification's bits
-  const long long W = g.R * g.wr;  // < 2^27 for grids below 2^31 points
-  const long long groups = (W + 3) / 4;
-  const long long dy = g.nx, dz = (long long)g.nx * g.ny;
-  for (long long q4 = (long long)blockIdx.x * blockDim.x + threadIdx.x; q4 < groups;
-       q4 += (long long)gridDim.x * blockDim.x) {
-    const long long w0 = 4 * q4;
-    int m, j, k;
-    const unsigned r = split_word(g, (unsigned)w0, m);
-    split_row(g, r, j, k);
-    uint32_t K[4] = {0u, 0u, 0u, 0u};
-    if (m + 4 <= g.wr) {  // four words of one row
-      if (j + 1 < g.ny && k + 1 < g.nz) {
-        const long long pos = (long long)r * g.nx + 32ll * m;
-        uint32_t a[4], a1[4], b[4], b1[4], c[4], c1[4], d[4], d1[4];
-        row_windows4(bits, pos, a, a1);
-        row_windows4(bits, pos + dy, b, b1);
-        row_windows4(bits, pos + dz, c, c1);
-        row_windows4(bits, pos + dy + dz, d, d1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          K[q] = a[q] & a1[q] & b[q] & b1[q] & c[q] & c1[q] & d[q] & d1[q] &
-                 low_mask(g.nx - 1 - 32 * (m + q));
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (w0 + q < W) K[q] = kept_word(g, bits, (uint32_t)(w0 + q));
-    }
-    if (w0 + 4 <= W) {
-      *reinterpret_cast<uint4*>(kept + w0) = make_uint4(K[0], K[1], K[2], K[3]);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (w0 + q < W) kept[w0 + q] = K[q];
-    }
-  }
-}
-
-// Used mask of point-row word w = (row r = (j, k), word m): the OR of the
-// kept masks of cell rows (j - 1 .. j, k - 1 .. k), each with its +x
-// neighbour cell.
-__device__ __forceinline__ uint32_t used_word(const Grid& g, const uint32_t* __restrict__ kept,
-                                              uint32_t w, uint32_t m, uint32_t j, uint32_t k) {
-  const uint32_t wy = (uint32_t)g.wr, wz = (uint32_t)g.wr * (uint32_t)g.ny;
-  uint32_t u = 0u;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {  // cell rows (j - (c & 1), k - (c >> 1))
-    const uint32_t cj = c & 1, ck = c >> 1;
-    if (j < cj || k < ck) continue;
-    const uint32_t wq = w - cj * wy - ck * wz;
-    const uint32_t K = __ldg(kept + wq);
-    const uint32_t Kp = m > 0 ? __ldg(kept + wq - 1) : 0u;
-    u |= K | (K << 1) | (Kp >> 31);
-  }
-  return u & low_mask(g.nx - 32 * (int)m);
-}
-
-// K2a, second pass: one 256-thread block per tile of kScanTile words
-// (grid-stride over tiles), thread t taking the 4-word groups t + 256 e:
-// used masks, packed counts and tile totals.
-__global__ void __launch_bounds__(256) k_thr_used(Grid g, const uint32_t* __restrict__ kept,
-                                                  uint32_t* __restrict__ used,
-                                                  uint32_t* __restrict__ wc,
-                                                  uint32_t* __restrict__ tile_tot, int tiles) {
-  __shared__ uint32_t s_red[24];
-  pdl_trigger();
-  pdl_wait();  // the kept masks
-  const long long W = g.R * g.wr;
-  const uint32_t wy = (uint32_t)g.wr, wz = (uint32_t)g.wr * (uint32_t)g.ny;
+  const int lane = threadIdx.x & 31;
+  const unsigned W = (unsigned)(g.R * g.wr), wr = (unsigned)g.wr, nx = (unsigned)g.nx;
+  const unsigned dz = nx * (unsigned)g.ny;
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned lo = (unsigned)tile * kScanTile, n = min((unsigned)kScanTile, W - lo);
+    const unsigned r0 = div_by(lo, g.mwr), rows = div_by(lo + n - 1u, g.mwr) - r0 + 1u;
+    // the fewest rows a lane with which the block covers the tile at once
+    const unsigned fit = kWarps * kCols / wr;
+    const unsigned depth = (rows + fit - 1u) / fit;
+    const unsigned items = (rows + depth - 1u) / depth * wr;
     uint32_t sk = 0, su = 0, sa = 0;
-#pragma unroll 1
-    for (int e = 0; e < kScanItems / 4; ++e) {
-      const long long w0 = (long long)tile * kScanTile + 4ll * (threadIdx.x + 256 * e);
-      if (w0 >= W) break;
-      int mi, ji, ki;
-      const uint32_t r = split_word(g, (uint32_t)w0, mi);
-      split_row(g, r, ji, ki);
-      const uint32_t m = (uint32_t)mi, j = (uint32_t)ji, k = (uint32_t)ki;
-      uint32_t own[4] = {0u, 0u, 0u, 0u}, U[4] = {0u, 0u, 0u, 0u};
-      if (m + 4 <= wy) {  // four words of one row: 5 kept words per cell row
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {  // cell rows (j - (c & 1), k - (c >> 1))
-          const uint32_t cj = c & 1, ck = c >> 1;
-          if (j < cj || k < ck) continue;
-          const uint32_t wq = (uint32_t)w0 - cj * wy - ck * wz;
-          uint32_t K[5];
-          K[0] = m > 0 ? __ldg(kept + wq - 1) : 0u;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) K[q + 1] = __ldg(kept + wq + q);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) U[q] |= K[q + 1] | (K[q + 1] << 1) | (K[q] >> 31);
-          if (c == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) own[q] = K[q + 1];
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) U[q] &= low_mask(g.nx - 32 * (int)(m + q));
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const long long w = w0 + q;
-          if (w >= W) break;
-          int mq, jq, kq;
-          const uint32_t rq = split_word(g, (uint32_t)w, mq);
-          split_row(g, rq, jq, kq);
-          own[q] = __ldg(kept + w);
-          U[q] = used_word(g, kept, (uint32_t)w, (uint32_t)mq, (uint32_t)jq, (uint32_t)kq);
-        }
+    for (unsigned q0 = (threadIdx.x >> 5) * kCols; q0 < items; q0 += kWarps * kCols) {
+      const unsigned q1 = q0 + (unsigned)lane;  // the lane's item, plus one
+      const bool mine = lane > 0 && q1 <= items;
+      const unsigned q = q1 == 0u ? 0u : min(q1 - 1u, items - 1u);
+      const unsigned chunk = div_by(q, g.mwr), m = q - chunk * wr;
+      const unsigned r = r0 + chunk * depth;
+      int j, k;
+      split_row(g, r, j, k);
+      unsigned pos = r * nx + 32u * m;
+      unsigned w = mine ? r * wr + m - lo : 0x80000000u;  // the word's place in the tile; before it: above n
+      const uint32_t cmask = low_mask(g.nx - 1 - 32 * (int)m), pmask = low_mask(g.nx - 32 * (int)m);
+      uint2 cur = plane_pairs(bits, pos, dz, k, g.nz);
+      uint32_t up = 0u;  // kept cells of cell row j - 1, of both planes
+      if (j > 0) {
+        const uint2 prev = plane_pairs(bits, pos - nx, dz, k, g.nz);
+        up = ((prev.x & cur.x) | (prev.y & cur.y)) & cmask;
       }
-      uint32_t pk[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        pk[q] = (uint32_t)__popc(own[q]) << 16 | (uint32_t)__popc(U[q]);
-        sk += pk[q] >> 16;
-        su += pk[q] & 0xffffu;
-        sa += pk[q] ? 1u : 0u;
-      }
-      if (w0 + 4 <= W) {
-        *reinterpret_cast<uint4*>(used + w0) = make_uint4(U[0], U[1], U[2], U[3]);
-        *reinterpret_cast<uint4*>(wc + w0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (w0 + q < W) {
-            used[w0 + q] = U[q];
-            wc[w0 + q] = pk[q];
-          }
+#pragma unroll 2
+      for (unsigned d = 0; d < depth; ++d) {
+        const bool cells = j + 1 < g.ny;  // the row has cells in y
+        j = cells ? j + 1 : 0;
+        k += cells ? 0 : 1;
+        pos += nx;
+        const uint2 nxt = plane_pairs(bits, pos, dz, k, g.nz);
+        const uint32_t own = cells ? nxt.y & cur.y & cmask : 0u;
+        const uint32_t dp = cells ? own | (nxt.x & cur.x & cmask) : 0u;
+        const uint32_t K = up | dp;
+        const uint32_t before = __shfl_up_sync(kFull, K, 1) >> 31;
+        const uint32_t U = (K | (K << 1) | (m > 0 ? before : 0u)) & pmask;
+        if (w < n) {
+          const uint32_t ck = __popc(own), cu = __popc(U);
+          used[lo + w] = U;
+          if (U) kept[lo + w] = own;
+          wc[lo + w] = ck << 16 | cu;
+          sk += ck;
+          su += cu;
+          sa += U ? 1u : 0u;
+        }
+        up = dp;
+        cur = nxt;
+        w += wr;
       }
     }
-    block_sum3(sk, su, sa, s_red);
-    if (threadIdx.x == 0) {
-      tile_tot[tile] = sk;
-      tile_tot[tiles + tile] = su;
-      tile_tot[2 * tiles + tile] = sa;
+    sk = __reduce_add_sync(kFull, sk);
+    su = __reduce_add_sync(kFull, su);
+    sa = __reduce_add_sync(kFull, sa);
+    if (lane == 0) {
+      atomicAdd(&s_sum[0], sk);
+      atomicAdd(&s_sum[1], su);
+      atomicAdd(&s_sum[2], sa);
     }
+    __syncthreads();
+    if (threadIdx.x < 3) tile_tot[threadIdx.x * tiles + tile] = s_sum[threadIdx.x];
+    __syncthreads();  // s_sum is free
   }
 }
 
 void launch_thr_count(const Grid& g, const uint32_t* bits, uint32_t* kept, uint32_t* used,
                       uint32_t* wc, uint32_t* tile_tot, int num_sms, cudaStream_t s) {
-  const long long W = g.R * g.wr;
-  const int b1 = resident_blocks(k_thr_kept, 256, 0, num_sms, (W + 1023) / 1024);
-  launch_pdl(k_thr_kept, (unsigned)b1, 256u, 0, s, g, bits, kept);
-  const int tiles = word_scan_tiles(W);
-  const int b2 = resident_blocks(k_thr_used, 256, 0, num_sms, tiles);
-  launch_pdl(k_thr_used, (unsigned)b2, 256u, 0, s, g, kept, used, wc, tile_tot, tiles);
+  (void)num_sms;
+  const int tiles = word_scan_tiles(g.R * g.wr);  // a block a tile
+  launch_pdl(k_thr_words, (unsigned)tiles, (unsigned)kThrThreads, 0, s, g, bits, kept, used, wc,
+             tile_tot, tiles);
 }
 
 // Words a warp of the emit takes at a time.  Small batches even the warps out:
