@@ -30,6 +30,7 @@
 #include "kernels.cuh"
 #include "mc_case.cuh"
 #include "mt_tables.h"
+#include "tma.cuh"
 
 namespace daxgb {
 
@@ -106,60 +107,198 @@ __device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_warp, uns
   return before + x - v;
 }
 
-// Warp w of a tile takes the kMtChunk consecutive cells of chunk 8 * tile + w
-// (lanes interleaved, so every load of ids is 512 contiguous bytes); the
-// chunk's and the tile's triangle totals are stored.
+// Warp w of a tile takes the kMtChunk consecutive cells of chunk 8 * tile + w;
+// the chunk's and the tile's triangle totals are stored.
 //
-// 83 million cells take 280 us, 1.33 GB of connectivity at 4.7 TB/s: the
-// gathers of a row of 32 cells touch 4 to 8 lines each, which L1 looks up one
-// at a time.  (The ids of two, four or eight cells loaded ahead of their
-// gathers took 310, 300 and 400 us.)
+// Bound by the connectivity's bytes (16 a cell): 83 million cells take 226 us,
+// 1.44 GB at 6.4 TB/s.  A bulk copy brings the ids of kMtGroup cells into the
+// warp's buffer, and as soon as they are in registers the next group's is issued,
+// also over the end of a tile.  A lane takes kMtRun consecutive cells: in a mesh of
+// tetrahedralized voxels, five cells each, the lanes then gather the same corner
+// of consecutive voxels, one or two lines a load.  The twenty ids of a lane are
+// checked by one unsigned maximum and their gathers issued together; a warp whose
+// cells reach past the end or list a bad id goes cell by cell.
+//
+// If the lanes' runs lie apart, more than half of them over 32 ids from the run
+// before, the lanes take consecutive cells instead, which then share lines within
+// a voxel: 471 us for voxels in random order, 683 by runs.
+//
+// (A cell a lane, with loads straight from global memory, touched 4 to 8 lines a
+// gather, which L1 looks up one at a time: 276 us, and 543 for voxels in random
+// order.  Runs with a check a cell were issue bound, 81 instructions a row of 32
+// cells: 292.  Two buffers a warp took as long, but left the gathers half the L1:
+// 2040 us for cells in no order at all, now 1280; the one order for which a cell a
+// lane was faster, 1080.)
+//
+// Connectivity that is not 16-byte aligned is copied by plain loads: 377 us.
+constexpr int kMtRun = 5;
+constexpr int kMtGroup = 32 * kMtRun;
+constexpr int kMtGroups = kMtChunk / kMtGroup;  // whole groups a chunk; the rest a cell a lane
+static_assert(kMtGroups == 3 && kMtChunk - kMtGroups * kMtGroup == 32,
+              "four groups a tile, the last of one cell a lane");
+
 template <bool VEC>
-__global__ void __launch_bounds__(kMtThreads) k_mt_count(const int32_t* __restrict__ conn,
-                                                         long long C,
-                                                         const float* __restrict__ f, long long P,
-                                                         float iso, uint8_t* __restrict__ cases,
-                                                         unsigned* __restrict__ tile_tot,
-                                                         unsigned* __restrict__ chunk_tot,
-                                                         Info* info, int tiles) {
-  __shared__ unsigned s_warp[kMtThreads / 32];
+__global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
+    k_mt_count(const int32_t* __restrict__ conn, long long C, const float* __restrict__ f,
+               long long P, float iso, uint8_t* __restrict__ cases, unsigned* __restrict__ tile_tot,
+               unsigned* __restrict__ chunk_tot, Info* info, int tiles) {
+  constexpr int kWarps = kMtThreads / 32;
+  __shared__ unsigned s_warp[2][kWarps];
+  __shared__ __align__(16) int4 s_ids[kWarps][kMtGroup];
+  __shared__ __align__(16) uint8_t s_case[kWarps][kMtChunk];
+  __shared__ uint64_t s_bar[kWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  bool bad = false;
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    unsigned sum = 0;
-    const long long cb = (long long)tile * kMtTile + (long long)wid * kMtChunk + lane;
-#pragma unroll 4
-    for (int r = 0; r < kMtChunk / 32; ++r) {
-      const long long c = cb + 32 * r;
-      if (c < C) {
-        int id[4];
-        int cs = 0;
-        if (load_tet<VEC>(conn, c, P, id)) {
-          const float v[4] = {__ldg(f + id[0]), __ldg(f + id[1]), __ldg(f + id[2]),
-                              __ldg(f + id[3])};
-          cs = mt_classify(v, iso);
+  uint8_t* const cs_of = s_case[wid];
+  if (VEC && lane == 0) {
+    mbar_init(&s_bar[wid], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  bool bad = false, late = false;
+  // an id is a point if it is below this as an unsigned: negative ones are not
+  const unsigned points = (unsigned)min(P, 1ll << 31);
+  unsigned long long policy = 0;
+  if (VEC) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  // the ids of group g of a tile's chunk into the warp's buffer
+  auto copy = [&](long long tile, int g) {
+    if (tile >= tiles || late) return;
+    const long long c = tile * kMtTile + (long long)wid * kMtChunk + g * kMtGroup;
+    const int n = (int)min((long long)(g < kMtGroups ? kMtGroup : 32), max(C - c, 0ll));
+    int4* dst = s_ids[wid];
+    if (VEC) {
+      if (lane == 0) {
+        uint64_t* bar = &s_bar[wid];
+        if (n > 0) {
+          mbar_arrive_tx(bar, 16u * n);
+          bulk_load(dst, conn + 4 * c, 16u * n, bar, policy);
         } else {
-          bad = true;
+          mbar_arrive(bar);
         }
-        cases[c] = (uint8_t)cs;
-        sum += (unsigned)mt_faces(cs);
       }
+    } else {
+      for (int i = lane; i < n; i += 32) {
+        const int32_t* q = conn + 4 * (c + i);
+        dst[i] = make_int4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+      }
+    }
+  };
+  auto landed = [&](int g) {  // four groups a tile: group g is of parity g & 1
+    if (VEC && !late) {
+      Spin sp;
+      bool ok;
+      while (!(ok = mbar_test(&s_bar[wid], g & 1)) && sp.more()) {
+      }
+      late = __any_sync(kFull, !ok);
+    }
+    __syncwarp();
+  };
+  auto classify = [&](const int4& q) -> int {
+    const bool ok = q.x >= 0 && (long long)q.x < P && q.y >= 0 && (long long)q.y < P && q.z >= 0 &&
+                    (long long)q.z < P && q.w >= 0 && (long long)q.w < P;
+    bad = bad || !ok;
+    if (!ok) return 0;
+    const float v[4] = {__ldg(f + q.x), __ldg(f + q.y), __ldg(f + q.z), __ldg(f + q.w)};
+    return mt_classify(v, iso);
+  };
+  copy(blockIdx.x, 0);
+  int flip = 0;
+#pragma unroll 1
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, flip ^= 1) {
+    unsigned sum = 0;
+    const long long cb = tile * kMtTile + (long long)wid * kMtChunk;
+#pragma unroll 1
+    for (int g = 0; g < kMtGroups; ++g) {
+      landed(g);
+      if (late) break;
+      const int4* ids = s_ids[wid];
+      int4 q[kMtRun];
+      int first = kMtRun * lane, step = 1;  // the lane's cells of the group
+      q[0] = ids[first];
+      const int before = __shfl_up_sync(kFull, q[0].x, 1);
+      if (__popc(__ballot_sync(kFull, (unsigned)(q[0].x - before + 32) > 64u)) > 16) {
+        first = lane;
+        step = 32;
+        q[0] = ids[first];
+      }
+      unsigned top = max(max((unsigned)q[0].x, (unsigned)q[0].y),
+                         max((unsigned)q[0].z, (unsigned)q[0].w));
+#pragma unroll
+      for (int i = 1; i < kMtRun; ++i) {
+        q[i] = ids[first + i * step];
+        top = max(max(top, max((unsigned)q[i].x, (unsigned)q[i].y)),
+                  max((unsigned)q[i].z, (unsigned)q[i].w));
+      }
+      const int at = g * kMtGroup + first;
+      // Whether every lane's ids are points.  The vote takes each lane's loaded
+      // values, so all of the loads have returned before the buffer is filled
+      // again (a barrier alone lets the copy pass loads that still wait).
+      const bool fast = __all_sync(kFull, top < points && cb + at + (kMtRun - 1) * step < C);
+      __syncwarp();
+      copy(tile, g + 1);
+      if (fast) {
+        float v[kMtRun][4];
+#pragma unroll
+        for (int i = 0; i < kMtRun; ++i) {
+          v[i][0] = __ldg(f + q[i].x);
+          v[i][1] = __ldg(f + q[i].y);
+          v[i][2] = __ldg(f + q[i].z);
+          v[i][3] = __ldg(f + q[i].w);
+        }
+#pragma unroll
+        for (int i = 0; i < kMtRun; ++i) {
+          const int cs = mt_classify(v[i], iso);
+          cs_of[at + i * step] = (uint8_t)cs;
+          sum += (unsigned)mt_faces(cs);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kMtRun; ++i) {
+          const int cs = cb + at + i * step < C ? classify(q[i]) : 0;
+          cs_of[at + i * step] = (uint8_t)cs;
+          sum += (unsigned)mt_faces(cs);
+        }
+      }
+    }
+    landed(kMtGroups);
+    if (!late) {
+      const int at = kMtGroups * kMtGroup + lane;
+      const int4 q = s_ids[wid][lane];
+      bool is = (unsigned)q.x < points && (unsigned)q.y < points && (unsigned)q.z < points &&
+                (unsigned)q.w < points;
+      bad = __any_sync(kFull, cb + at < C && !is) || bad;  // as above, every load has returned
+      __syncwarp();
+      copy(tile + gridDim.x, 0);
+      is = is && cb + at < C;
+      int cs = 0;
+      if (is) {
+        const float v[4] = {__ldg(f + q.x), __ldg(f + q.y), __ldg(f + q.z), __ldg(f + q.w)};
+        cs = mt_classify(v, iso);
+      }
+      cs_of[at] = (uint8_t)cs;
+      sum += (unsigned)mt_faces(cs);
+    }
+    __syncwarp();
+    // the chunk's cases in whole lines
+    if (cb + kMtChunk <= C && (reinterpret_cast<uintptr_t>(cases) & 15) == 0) {
+      reinterpret_cast<uint4*>(cases + cb)[lane] = reinterpret_cast<const uint4*>(cs_of)[lane];
+    } else {
+      for (int i = lane; i < kMtChunk && cb + i < C; i += 32) cases[cb + i] = cs_of[i];
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
     if (lane == 0) {
-      chunk_tot[(long long)tile * (kMtTile / kMtChunk) + wid] = sum;
-      s_warp[wid] = sum;
+      chunk_tot[tile * (kMtTile / kMtChunk) + wid] = sum;
+      s_warp[flip][wid] = sum;
     }
-    __syncthreads();
+    __syncthreads();  // one a tile: s_warp's other row is written before the next one
     if (threadIdx.x == 0) {
       unsigned t = 0;
-      for (int w = 0; w < kMtThreads / 32; ++w) t += s_warp[w];
+      for (int w = 0; w < kWarps; ++w) t += s_warp[flip][w];
       tile_tot[tile] = t;
     }
-    __syncthreads();
   }
   if (bad) atomicOr(&info->error, kErrBadIndex);
+  if (late) atomicOr(&info->error, kErrTimeout);
 }
 
 // One block: exclusive offsets of the tile totals (tile_off[tiles] = T) and
