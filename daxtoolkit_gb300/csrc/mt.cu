@@ -130,7 +130,7 @@ __device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_warp, uns
 // 2040 us for cells in no order at all, now 1280; the one order for which a cell a
 // lane was faster, 1080.)
 //
-// Connectivity that is not 16-byte aligned is copied by plain loads: 377 us.
+// Connectivity that is not 16-byte aligned is copied by plain loads: 376 us, as before.
 constexpr int kMtRun = 5;
 constexpr int kMtGroup = 32 * kMtRun;
 constexpr int kMtGroups = kMtChunk / kMtGroup;  // whole groups a chunk; the rest a cell a lane
@@ -231,8 +231,10 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
       const int at = g * kMtGroup + first;
       // Whether every lane's ids are points.  The vote takes each lane's loaded
       // values, so all of the loads have returned before the buffer is filled
-      // again (a barrier alone lets the copy pass loads that still wait).
+      // again (a barrier alone lets the copy pass loads that still wait); the fence
+      // orders them before the copy's writes.
       const bool fast = __all_sync(kFull, top < points && cb + at + (kMtRun - 1) * step < C);
+      if (VEC) fence_proxy_async();
       __syncwarp();
       copy(tile, g + 1);
       if (fast) {
@@ -266,6 +268,7 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
       bool is = (unsigned)q.x < points && (unsigned)q.y < points && (unsigned)q.z < points &&
                 (unsigned)q.w < points;
       bad = __any_sync(kFull, cb + at < C && !is) || bad;  // as above, every load has returned
+      if (VEC) fence_proxy_async();
       __syncwarp();
       copy(tile + gridDim.x, 0);
       is = is && cb + at < C;
