@@ -730,6 +730,18 @@ int dax_gb300_mt_count(const int32_t* d_conn, int64_t num_cells, const float* d_
   return check_launch("marching tetrahedra count kernels");
 }
 
+int dax_gb300_selfcheck_mt_wait(const int32_t* d_conn, int64_t num_cells, const float* d_field,
+                                int64_t num_points, float isovalue, void* d_scratch,
+                                size_t scratch_bytes, void* stream) {
+  int st = mt_args(d_conn, num_cells, d_field, num_points, d_scratch, scratch_bytes);
+  if (st) return st;
+  if (num_cells == 0) return fail(DAX_GB300_ERROR_BAD_VALUE, "no cells, no wait");
+  daxgb::launch_mt_count(d_conn, num_cells, d_field, num_points, isovalue,
+                         static_cast<char*>(d_scratch), num_sms(),
+                         static_cast<cudaStream_t>(stream), 0);
+  return check_launch("marching tetrahedra count kernels");
+}
+
 int dax_gb300_mt_classify_count(const int32_t* d_conn, int64_t num_cells, const float* d_field,
                                 int64_t num_points, float isovalue, int32_t* d_count,
                                 void* stream) {

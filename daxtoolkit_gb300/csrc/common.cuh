@@ -19,6 +19,7 @@
 namespace daxgb {
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr unsigned kSpinIters = 1u << 24;  // the most polls of a bounded wait
 
 // Host-prepared, device-consumed description of one uniform grid.
 struct Grid {

@@ -389,8 +389,10 @@ MtLayout mt_layout(long long C);
 // Bits of the B half of a merge key (A << bits) | B: P <= 2^bits.  Keys are
 // 32-bit when 2 * bits <= 32, else 64-bit.
 int mt_key_bits(long long P);
+// polls: the most polls of a wait for connectivity in flight (0: every such
+// wait runs out at once).
 void launch_mt_count(const int32_t* conn, long long C, const float* f, long long P, float iso,
-                     char* scratch, int num_sms, cudaStream_t s);
+                     char* scratch, int num_sms, cudaStream_t s, unsigned polls = kSpinIters);
 void launch_mt_cell_count(const int32_t* conn, long long C, const float* f, long long P,
                           float iso, int32_t* count, int* err, int num_sms, cudaStream_t s);
 void launch_mt_emit_direct(const float* pts, const int32_t* conn, long long C, const float* f,

@@ -141,7 +141,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
     k_mt_count(const int32_t* __restrict__ conn, long long C, const float* __restrict__ f,
                long long P, float iso, uint8_t* __restrict__ cases, unsigned* __restrict__ tile_tot,
-               unsigned* __restrict__ chunk_tot, Info* info, int tiles) {
+               unsigned* __restrict__ chunk_tot, Info* info, int tiles, unsigned polls) {
   constexpr int kWarps = kMtThreads / 32;
   __shared__ unsigned s_warp[2][kWarps];
   __shared__ __align__(16) int4 s_ids[kWarps][kMtGroup];
@@ -154,7 +154,8 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
-  bool bad = false, late = false;
+  bool bad = false, late = false;  // late: a copy did not land in time, and no other is issued
+  int awaited = 0;                 // its group
   // an id is a point if it is below this as an unsigned: negative ones are not
   const unsigned points = (unsigned)min(P, 1ll << 31);
   unsigned long long policy = 0;
@@ -184,11 +185,11 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
   };
   auto landed = [&](int g) {  // four groups a tile: group g is of parity g & 1
     if (VEC && !late) {
-      Spin sp;
-      bool ok;
-      while (!(ok = mbar_test(&s_bar[wid], g & 1)) && sp.more()) {
-      }
+      Spin sp(polls);
+      bool ok = polls > 0 && mbar_test(&s_bar[wid], g & 1);
+      while (!ok && sp.more()) ok = mbar_test(&s_bar[wid], g & 1);
       late = __any_sync(kFull, !ok);
+      awaited = g;
     }
     __syncwarp();
   };
@@ -301,7 +302,12 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
     }
   }
   if (bad) atomicOr(&info->error, kErrBadIndex);
-  if (late) atomicOr(&info->error, kErrTimeout);
+  if (late) {
+    atomicOr(&info->error, kErrTimeout);
+    Spin sp;
+    while (!mbar_test(&s_bar[wid], awaited & 1) && sp.more()) {
+    }
+  }
 }
 
 // One block: exclusive offsets of the tile totals (tile_off[tiles] = T) and
@@ -948,7 +954,7 @@ int mt_key_bits(long long P) {
 }
 
 void launch_mt_count(const int32_t* conn, long long C, const float* f, long long P, float iso,
-                     char* scratch, int num_sms, cudaStream_t s) {
+                     char* scratch, int num_sms, cudaStream_t s, unsigned polls) {
   const MtLayout L = mt_layout(C);
   Info* info = reinterpret_cast<Info*>(scratch + L.info);
   cudaMemsetAsync(info, 0, sizeof(Info), s);
@@ -958,11 +964,12 @@ void launch_mt_count(const int32_t* conn, long long C, const float* f, long long
   unsigned* ctot = reinterpret_cast<unsigned*>(scratch + L.chunk_tot);
   if (vec) {
     const int b = resident_blocks(k_mt_count<true>, kMtThreads, 0, num_sms, L.tiles);
-    k_mt_count<true><<<b, kMtThreads, 0, s>>>(conn, C, f, P, iso, cases, tot, ctot, info, L.tiles);
+    k_mt_count<true><<<b, kMtThreads, 0, s>>>(conn, C, f, P, iso, cases, tot, ctot, info, L.tiles,
+                                              polls);
   } else {
     const int b = resident_blocks(k_mt_count<false>, kMtThreads, 0, num_sms, L.tiles);
     k_mt_count<false><<<b, kMtThreads, 0, s>>>(conn, C, f, P, iso, cases, tot, ctot, info,
-                                               L.tiles);
+                                               L.tiles, polls);
   }
   k_mt_tile_scan<<<1, 1024, 0, s>>>(tot, L.tiles,
                                     reinterpret_cast<unsigned long long*>(scratch + L.tile_off),

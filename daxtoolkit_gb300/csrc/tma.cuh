@@ -3,10 +3,10 @@
 // other blocks.
 #pragma once
 #include <cstdint>
+#include "common.cuh"
 
 namespace daxgb {
 
-constexpr unsigned kSpinIters = 1u << 24;
 constexpr unsigned long long kSpinNs = 200000000ull;  // 0.2 s
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -84,15 +84,18 @@ __device__ __forceinline__ void bulk_store_and_wait_read(void* dst, const void* 
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
-// Bounded waiting: more() is false once kSpinIters polls or kSpinNs have
-// passed since the first poll.
+// Bounded waiting: more() is false once `polls` polls or kSpinNs have passed
+// since the first poll.  A wait that runs out with a copy into the block's
+// shared memory in flight waits once more, with the default limit, before the
+// block leaves: the copy would land in memory that is another block's by then.
 struct Spin {
-  unsigned n = 0;
+  unsigned n = 0, polls;
   unsigned long long t0 = 0;
+  __device__ __forceinline__ explicit Spin(unsigned polls = kSpinIters) : polls(polls) {}
   __device__ __forceinline__ bool more() {
     if (n == 0) t0 = now_ns();
     ++n;
-    if (n >= kSpinIters) return false;
+    if (n >= polls) return false;
     if ((n & 63u) == 0u && now_ns() - t0 > kSpinNs) return false;
     return true;
   }

@@ -43,10 +43,12 @@ typedef enum dax_gb300_status {
   DAX_GB300_ERROR_CUDA = 4,
   /* an output buffer is smaller than the result; nothing was written */
   DAX_GB300_ERROR_CAPACITY = 5,
-  /* a bounded device-side wait gave up (the fused count pass's blocks wait
-     on one another); the count pass has no result and the generate pass writes nothing.  The single-pass
-     integer scan, StreamCompact and Unique (whose tiles wait on the sums of
-     earlier tiles) report it when their total or count is read */
+  /* a bounded device-side wait gave up: the fused count pass's blocks wait on
+     one another, the marching tetrahedra count on its copies of the
+     connectivity; the count pass then has no result and the generate pass
+     writes nothing.  The single-pass integer scan, StreamCompact and Unique
+     (whose tiles wait on the sums of earlier tiles) report it when their total
+     or count is read */
   DAX_GB300_ERROR_TIMEOUT = 6,
   /* grid shape outside what the kernels support (see each call) */
   DAX_GB300_ERROR_UNSUPPORTED = 7
@@ -124,6 +126,14 @@ int dax_gb300_mc_pipeline_plan(const dax_gb300_uniform_grid* grid, int slabs, in
 int dax_gb300_selfcheck_division(const float* d_divisors, int num_divisors, uint32_t first,
                                  uint64_t count, uint32_t step, unsigned long long* d_mismatches,
                                  void* stream);
+
+/* Self-check of the marching tetrahedra count's give-up path:
+ * dax_gb300_mt_count with waits for the connectivity that run out at once.
+ * On a 16-byte boundary the totals are then DAX_GB300_ERROR_TIMEOUT and a
+ * generate pass writes nothing; other connectivity is not waited for. */
+int dax_gb300_selfcheck_mt_wait(const int32_t* d_conn, int64_t num_cells, const float* d_field,
+                                int64_t num_points, float isovalue, void* d_scratch,
+                                size_t scratch_bytes, void* stream);
 const char* dax_gb300_last_error(void);
 
 /* Sets the message dax_gb300_last_error() returns on this thread and returns
