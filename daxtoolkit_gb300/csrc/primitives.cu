@@ -264,9 +264,11 @@ void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, voi
 // Tiles are taken in ticket order and each block's tickets increase in the
 // order it processes them, so the smallest unfinished tile always has all
 // its predecessors' sums published and its block working on it: no tile
-// waits on a later one.  Every wait is still bounded (Spin), and a wait that
-// runs out marks the scan failed (DAX_GB300_ERROR_TIMEOUT when the total is
-// read).
+// waits on a later one.  Every wait is still bounded (Spin).  A wait that runs
+// out marks the scan failed (DAX_GB300_ERROR_TIMEOUT when the total is read),
+// and nothing is written for a tile whose prefix is not known: the look-back
+// warp publishes such a tile as BAD, which ends the look-back of every later
+// tile that meets it, and compute warps without a prefix write no more tiles.
 //
 // Integer sums wrap, so any split of the look-back gives the same result;
 // float scans keep the deterministic reduce-then-scan above.
@@ -282,7 +284,7 @@ void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, voi
 // Scratch (zeroed before the launch, the states included): ticket, error,
 // total, then per tile its state: flag << 32 | sum in one 64-bit word for
 // 32-bit sums, two such words (low and high halves) for 64-bit sums.
-constexpr unsigned kStAgg = 1u, kStInc = 2u;
+constexpr unsigned kStAgg = 1u, kStInc = 2u, kStBad = 3u;
 constexpr size_t kScanHead = 64;
 constexpr int kSThreads = 512;  // compute threads
 constexpr int kSElems = 8192;   // elements a tile
@@ -371,34 +373,37 @@ __device__ __forceinline__ A warp_inclusive(A x, int lane) {
 // The exclusive prefix of `tile` from the states of the tiles before it
 // (one warp; every lane returns it).  A step reads the states of tiles
 // top - lane, polls those not yet published (a short sleep between polls),
-// and ends at the nearest inclusive prefix.  Sets `failed` if a wait ran out.
+// and ends at the nearest inclusive prefix.  Sets `failed` (on every lane) if
+// a wait ran out, here or before the nearest tile that knows.
 template <typename A>
-__device__ A look_back(const TileStates<A>& st, int tile, int lane, bool& failed) {
+__device__ A look_back(const TileStates<A>& st, int tile, int lane, unsigned polls, bool& failed) {
   A prefix = 0;
+  failed = false;
   for (int top = tile - 1; top >= 0; top -= 32) {
     const int t = top - lane;
     A x = 0;
     unsigned f = kStInc;  // before tile 0: an inclusive zero
     if (t >= 0) {
-      Spin spin;
+      Spin spin(polls);
       while ((f = st.read(t, x)) == 0u) {
         if (!spin.more()) {
-          failed = true;
-          f = kStInc;
-          x = 0;
+          f = kStBad;
           break;
         }
         __nanosleep(300);
       }
     }
-    // the nearest tile with its inclusive prefix ends the look-back
-    const unsigned incl = __ballot_sync(kFull, f == kStInc);
+    // the nearest tile with its inclusive prefix (or none) ends the look-back
+    const unsigned incl = __ballot_sync(kFull, f >= kStInc);
     const int last = incl ? __ffs(incl) - 1 : 31;
     A part = lane <= last ? x : (A)0;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(kFull, part, d);
     prefix += part;
-    if (incl) break;
+    if (incl) {
+      failed = __shfl_sync(kFull, f, last) == kStBad;
+      break;
+    }
   }
   return prefix;
 }
@@ -418,8 +423,9 @@ __device__ __forceinline__ bool compute_all(bool ok) {
   return all != 0;
 }
 
-__device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity) {
-  Spin sp;
+__device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity,
+                                           unsigned polls = kSpinIters) {
+  Spin sp(polls);
   while (!mbar_test(bar, parity))
     if (!sp.more()) return false;
   return true;
@@ -453,7 +459,7 @@ constexpr int kSBlock = kSThreads + 64;
 
 template <class Op>
 __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles, ScanCtl* ctl,
-                                            char* states, int bulk) {
+                                            char* states, int bulk, unsigned polls) {
   typedef typename Op::Staged Staged;
   typedef typename Op::Sum Sum;
   typedef typename Op::Carry Carry;
@@ -469,6 +475,7 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
   __shared__ int s_tile[kSStages];  // the stage's occupant
   __shared__ int s_seen[kSStages];  // the occupant as handed to the look-back warp
   __shared__ Sum s_tot[kSStages], s_pre[kSStages], s_wsum[kSStages][kWarps];
+  __shared__ bool s_known[kSStages];  // whether s_pre is the tile's prefix
   __shared__ unsigned long long s_aux[kSStages];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // a tile is copied in bulk when it is whole and the arrays are 16-byte aligned
@@ -480,7 +487,6 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
       mbar_init(&b_agg[k], 1);
       mbar_init(&b_pre[k], 1);
       mbar_init(&b_done[k], kWarps);
-      s_pre[k] = 0;  // a wait that runs out leaves a prefix that is never too large
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -495,7 +501,7 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
     // waits for the output of use i and stores it
     auto retire = [&](int i) {
       const int k = i % kSStages, t = s_tile[k];
-      ok = wait_phase(&b_done[k], (i / kSStages) & 1);
+      ok = wait_phase(&b_done[k], (i / kSStages) & 1, polls);
       if (ok && whole(t)) op.store(stage(k), (long long)t * kTileElems);
     };
     int i = 0;
@@ -529,17 +535,21 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
     // the look-back warp: the block's tiles in order
     for (int i = 0;; ++i) {
       const int k = i % kSStages;
-      bool failed = !wait_phase(&b_agg[k], (i / kSStages) & 1);
+      if (!__all_sync(kFull, wait_phase(&b_agg[k], (i / kSStages) & 1, polls))) {
+        if (lane == 0) atomicOr(&ctl->error, 1u);
+        break;
+      }
       const int tile = s_seen[k];
-      if (tile >= tiles || __any_sync(kFull, failed)) break;
+      if (tile >= tiles) break;
       const Sum tot = s_tot[k];
-      const Sum prefix = look_back(st, tile, lane, failed);
-      failed = __any_sync(kFull, failed);
+      bool failed;
+      const Sum prefix = look_back(st, tile, lane, polls, failed);
       if (lane == 0) {
-        if (tile > 0) st.publish(tile, kStInc, prefix + tot);
+        if (tile > 0) st.publish(tile, failed ? kStBad : kStInc, prefix + tot);
         if (failed) atomicOr(&ctl->error, 1u);
         if (tile == tiles - 1) ctl->total = (unsigned long long)(prefix + tot);
         s_pre[k] = prefix;
+        s_known[k] = !failed;
         mbar_arrive(&b_pre[k]);
       }
       __syncwarp();
@@ -554,7 +564,7 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
   auto reduce = [&](int i, Carry& carry) -> int {
     const int k = i % kSStages;
     int tile = tiles;
-    if (compute_all(wait_phase(&b_full[k], (i / kSStages) & 1)))
+    if (compute_all(wait_phase(&b_full[k], (i / kSStages) & 1, polls)))
       tile = s_tile[k];
     else if (threadIdx.x == 0)
       atomicOr(&ctl->error, 1u);
@@ -598,18 +608,25 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
     tile[d] = tiles;
     if (d == 0 || tile[d > 0 ? d - 1 : 0] < tiles) tile[d] = reduce(d, carry[d]);
   }
+  bool lost = false;  // the warp got no prefix for a tile: it only sums, for the block's barriers,
+                      // and the copy warp, whose stage does not come back, gives up
   for (int i = 0; tile[0] < tiles; ++i) {
     const int k = i % kSStages;
     tile[kAhead] = tile[kAhead - 1] < tiles ? reduce(i + kAhead, carry[kAhead]) : tiles;
-    wait_phase(&b_pre[k], (i / kSStages) & 1);  // a timeout is the look-back warp's to report
-    Sum run = s_pre[k];
-    for (int w = 0; w < warp; ++w) run += s_wsum[k][w];
-    op.finish(stage(k), (long long)tile[0] * kTileElems, run, warp, lane, carry[0], whole(tile[0]));
-    // the warp's shared-memory writes before the bulk copy reads them (and its
-    // reads before the stage's next bulk copy writes it)
-    fence_proxy_async();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&b_done[k]);
+    if (!lost && !__all_sync(kFull, wait_phase(&b_pre[k], (i / kSStages) & 1, polls) && s_known[k])) {
+      lost = true;
+      if (lane == 0) atomicOr(&ctl->error, 1u);
+    }
+    if (!lost) {
+      Sum run = s_pre[k];
+      for (int w = 0; w < warp; ++w) run += s_wsum[k][w];
+      op.finish(stage(k), (long long)tile[0] * kTileElems, run, warp, lane, carry[0], whole(tile[0]));
+      // the warp's shared-memory writes before the bulk copy reads them (and
+      // its reads before the stage's next bulk copy writes it)
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&b_done[k]);
+    }
 #pragma unroll
     for (int d = 0; d < kAhead; ++d) {
       tile[d] = tile[d + 1];
@@ -682,8 +699,9 @@ struct ScanPass {
 
 template <typename T>
 __global__ void __launch_bounds__(kSBlock, 1)
-    k_scan_single(ScanPass<T> op, long long n, int tiles, ScanCtl* ctl, char* states, int bulk) {
-  single_pass(op, n, tiles, ctl, states, bulk);
+    k_scan_single(ScanPass<T> op, long long n, int tiles, ScanCtl* ctl, char* states, int bulk,
+                  unsigned polls) {
+  single_pass(op, n, tiles, ctl, states, bulk, polls);
 }
 
 int single_pass_tiles(long long n) { return (int)((n + kSElems - 1) / kSElems); }
@@ -697,10 +715,13 @@ size_t single_scan_bytes(long long n) {
 // Clears the scratch's control words and tile states and launches one block
 // an SM of `kernel` (the ring is above the 48 KB of shared memory a launch
 // gets without opting in: set once per device and kernel; a failure shows
-// as the launch's error).
+// as the launch's error).  The self-check of the waits: polls, the most polls
+// of a wait; lost, whether no block takes tile 0, whose sum every other tile
+// then waits for in vain.
 template <class Op>
-void launch_single_pass(void (*kernel)(Op, long long, int, ScanCtl*, char*, int), const Op& op,
-                        long long n, int bulk, char* scratch, int num_sms, cudaStream_t s) {
+void launch_single_pass(void (*kernel)(Op, long long, int, ScanCtl*, char*, int, unsigned),
+                        const Op& op, long long n, int bulk, char* scratch, int num_sms,
+                        cudaStream_t s, unsigned polls = kSpinIters, bool lost = false) {
   typedef typename Op::Staged Staged;
   typedef typename Op::Sum Sum;
   const size_t smem = kSRing;
@@ -717,17 +738,18 @@ void launch_single_pass(void (*kernel)(Op, long long, int, ScanCtl*, char*, int)
   const int tiles = single_pass_tiles(n);
   const int blocks = tiles < num_sms ? tiles : num_sms;
   cudaMemsetAsync(scratch, 0, kScanHead + TileStates<Sum>::clear_bytes(tiles), s);
+  if (lost) cudaMemsetAsync(scratch, 1, 1, s);  // the first ticket is 1 (little-endian)
   kernel<<<blocks, kSBlock, smem, s>>>(op, n, tiles, reinterpret_cast<ScanCtl*>(scratch),
-                                              scratch + kScanHead, bulk);
+                                       scratch + kScanHead, bulk, polls);
 }
 
 template <typename T>
 void scan_single(const T* in, T* out, long long n, bool exclusive, char* scratch, int num_sms,
-                 cudaStream_t s) {
+                 cudaStream_t s, unsigned polls = kSpinIters, bool lost = false) {
   typedef typename Acc<T>::type A;
   const ScanPass<T> op{reinterpret_cast<const A*>(in), out, n, exclusive ? 1 : 0};
   const int bulk = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  launch_single_pass(k_scan_single<T>, op, n, bulk, scratch, num_sms, s);
+  launch_single_pass(k_scan_single<T>, op, n, bulk, scratch, num_sms, s, polls, lost);
 }
 
 // ---- radix sort -------------------------------------------------------------
@@ -1375,8 +1397,8 @@ struct CompactPass {
 template <typename S, int W, bool UNIQUE>
 __global__ void __launch_bounds__(kSBlock, 1)
     k_compact_single(CompactPass<S, W, UNIQUE> op, long long n, int tiles, ScanCtl* ctl,
-                     char* states, int bulk) {
-  single_pass(op, n, tiles, ctl, states, bulk);
+                     char* states, int bulk, unsigned polls) {
+  single_pass(op, n, tiles, ctl, states, bulk, polls);
 }
 
 template <typename S, int W, bool UNIQUE = false>
@@ -1566,14 +1588,14 @@ int read_back(void* host, const void* dev, size_t bytes, cudaStream_t s, const c
   return DAX_GB300_ERROR_CUDA;
 }
 
-// The element count of a single-pass compaction (synchronises the stream);
-// a look-back wait that ran out is DAX_GB300_ERROR_TIMEOUT.
+// The element count of a single-pass compaction, or the total of a scan
+// (synchronises the stream); a wait that ran out is DAX_GB300_ERROR_TIMEOUT.
 int read_count(int64_t* h_count, const char* scratch, cudaStream_t s, const char* what) {
   ScanCtl ctl;
   int st = read_back(&ctl, scratch, sizeof(ctl), s, what);
   if (st) return st;
   if (ctl.error) {
-    set_last_error(std::string(what) + ": a look-back wait expired on the device");
+    set_last_error(std::string(what) + ": a wait expired on the device");
     return DAX_GB300_ERROR_TIMEOUT;
   }
   *h_count = (int64_t)ctl.total;
@@ -1651,15 +1673,28 @@ int dax_gb300_scan(const void* d_in, void* d_out, int64_t n, int type, int exclu
   if (type == DAX_GB300_TYPE_F32)  // the scanned tile sums end with the grand total
     return read_back(h_total, sc + (size_t)ptiles(n) * tb, (size_t)tb, s, "reading the scan total");
   // the single pass: the error word and the total (little-endian, as wide as the element)
-  ScanCtl ctl;
-  st = read_back(&ctl, sc, sizeof(ctl), s, "reading the scan total");
-  if (st) return st;
-  if (ctl.error) {
-    set_last_error("scan: a look-back wait expired on the device");
-    return DAX_GB300_ERROR_TIMEOUT;
-  }
-  memcpy(h_total, &ctl.total, (size_t)tb);
-  return DAX_GB300_SUCCESS;
+  int64_t total = 0;
+  st = read_count(&total, sc, s, "reading the scan total");
+  if (!st) memcpy(h_total, &total, (size_t)tb);
+  return st;
+}
+
+int dax_gb300_selfcheck_scan_wait(const int32_t* d_in, int32_t* d_out, int64_t n, uint32_t polls,
+                                  int lost, void* d_scratch, size_t scratch_bytes, int32_t* h_total,
+                                  void* stream) {
+  using namespace daxgb;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!size_ok(n) || n <= kSElems) return bad("the scan must have two tiles or more");
+  if (!d_in || !d_out || !d_scratch || !h_total) return bad("NULL argument");
+  if (scratch_bytes < public_scan_bytes(n))
+    return bad("scratch smaller than dax_gb300_scan_scratch_bytes()");
+  scan_single<int32_t>(d_in, d_out, n, false, static_cast<char*>(d_scratch), prim_sms(), s,
+                       polls < kSpinIters ? polls : kSpinIters, lost != 0);
+  int st = launched("scan kernels");
+  int64_t total = 0;
+  if (!st) st = read_count(&total, static_cast<char*>(d_scratch), s, "reading the scan total");
+  if (!st) *h_total = (int32_t)total;
+  return st;
 }
 
 size_t dax_gb300_sort_scratch_bytes(int64_t n, int key_type, int value_bytes) {

@@ -134,6 +134,15 @@ int dax_gb300_selfcheck_division(const float* d_divisors, int num_divisors, uint
 int dax_gb300_selfcheck_mt_wait(const int32_t* d_conn, int64_t num_cells, const float* d_field,
                                 int64_t num_points, float isovalue, void* d_scratch,
                                 size_t scratch_bytes, void* stream);
+
+/* Self-check of the single-pass scan's bounded waits: an inclusive scan of
+ * more than 8192 int32 whose waits run out after `polls` polls, and with lost
+ * != 0 without its first tile, which every other tile waits for.  SUCCESS with
+ * the scan and its total, or DAX_GB300_ERROR_TIMEOUT with every element either
+ * right or as it was (lost: all as they were). */
+int dax_gb300_selfcheck_scan_wait(const int32_t* d_in, int32_t* d_out, int64_t n, uint32_t polls,
+                                  int lost, void* d_scratch, size_t scratch_bytes, int32_t* h_total,
+                                  void* stream);
 const char* dax_gb300_last_error(void);
 
 /* Sets the message dax_gb300_last_error() returns on this thread and returns
