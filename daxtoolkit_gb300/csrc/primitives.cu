@@ -1270,6 +1270,19 @@ struct CompactOp {
 // of one word.  (Testing the elements a second time and scanning each chunk
 // took 46 instructions a row of 32, from eight warps: 351 us for 100 M int32
 // and their values, 0.92 GB, now 185.)
+//
+// Values of two words and more leave a chunk (128 elements) at a time through
+// shared memory, consecutive lanes storing consecutive words: a lane that stores
+// its own elements' words covers a part of as many sectors as it stores words,
+// and with sixteen warps in turn few of them meet in L1: 20 M values of three words,
+// all kept, 85 M sector writes in L2 and 307 us, now 166; half of them kept, 156
+// and 133.  (At 60 M, a twentieth kept, it costs a little: 226 and 236 us; storing
+// such chunks from the lanes, behind a test, took 242.)
+template <int W>
+struct alignas(W == 4 ? 16 : W == 2 ? 8 : 4) Row {
+  uint32_t w[W];
+};
+
 template <typename S, int W, bool UNIQUE>
 struct CompactPass {
   typedef S Staged;
@@ -1368,8 +1381,26 @@ struct CompactPass {
                      all = __shfl_sync(kFull, incl, 31);
 #pragma unroll
       for (int g = 0; g < kG; ++g) {
+        const unsigned count = (all >> (8 * g)) & 0xffu;
+        if constexpr (W > 1) {
+          // through the warp's part of the staged stencil, which nothing reads again
+          Row<W>* const row = reinterpret_cast<Row<W>*>(lane_chunk0(s_data, warp, 0));
+          const uint32_t* const words = reinterpret_cast<const uint32_t*>(row);
+          const Row<W>* const v = reinterpret_cast<const Row<W>*>(vals[g]);
+          unsigned at = (before >> (8 * g)) & 0xffu;
+#pragma unroll
+          for (int e = 0; e < E; ++e)
+            if ((kept >> (g * E + e)) & 1u) row[at++] = v[e];
+          __syncwarp();
+          uint32_t* const dst = static_cast<uint32_t*>(out) + (unsigned long long)run * W;
+#pragma unroll 4
+          for (unsigned w = lane; w < count * W; w += 32) dst[w] = words[w];
+          __syncwarp();
+          run += count;
+          continue;
+        }
         unsigned long long pos = run + ((before >> (8 * g)) & 0xffu);
-        run += (all >> (8 * g)) & 0xffu;
+        run += count;
         Chunk x;
         if (UNIQUE) x = *reinterpret_cast<const Chunk*>(p + 32 * (c0 + g) * E);
         const long long i0 = wb + (32 * (c0 + g) + lane) * E;
