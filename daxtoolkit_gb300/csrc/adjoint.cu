@@ -59,8 +59,8 @@ __device__ __forceinline__ float width_z(const Grid& g, int k) {
 //
 // Bound by HBM.  Three strided loads a cell held in registers, no plane ahead,
 // in segments of 32 planes took 135 us for 385 x 321 x 289 (567 MB, 85 us at
-// the copy bandwidth), now 121, and 109 from a clean L2.  (4-byte copies, 73
-// instructions a row against 42, measured no faster than the loads.)
+// the copy bandwidth), now 103.  (4-byte copies, 73 instructions a row against
+// 42, measured no faster than the loads.)
 //
 // A block is one warp: the tile's place is then uniform over the block, and
 // the row addresses and tests are scalar work.
@@ -209,7 +209,7 @@ __device__ __forceinline__ void grad_adjoint_task(const Grid& g, const float* __
 
 __host__ __device__ inline int adj_nxw(const Grid& g) { return (g.nx + kMarchCols - 1) / kMarchCols; }
 __host__ __device__ inline int adj_bands(const Grid& g) { return (g.ny + kAdjBand - 1) / kAdjBand; }
-__host__ __device__ inline MarchTiles adj_set_tiles(const Grid& g, int seg) {
+__host__ __device__ inline MarchTiles adj_tiles(const Grid& g, int seg) {
   return march_tiles(adj_nxw(g), adj_bands(g), g.nz, (g.nz + seg - 1) / seg);
 }
 
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(32, kAdjMinBlocks)
                        const float* __restrict__ dg, float* __restrict__ out) {
   const int si = block_slot(block0, S.count, blockIdx.x);
   const Grid g = S.slots[si].g;
-  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0, adj_set_tiles(g, seg),
+  grad_adjoint_task(g, dg + 3 * S.slots[si].cell0, out + S.slots[si].point0, adj_tiles(g, seg),
                     (long long)blockIdx.x - __ldg(block0 + si));
 }
 
@@ -455,7 +455,7 @@ int adjoint_wave(int num_sms) {
   return resident_blocks(k_grad_adjoint_set, 32, kAdjSmem, num_sms, 1ll << 30);
 }
 long long adjoint_grad_blocks(const Grid& g, int seg) {
-  return adj_set_tiles(g, seg).tasks;
+  return adj_tiles(g, seg).tasks;
 }
 long long adjoint_edge_blocks(const Grid& g, int words) { return (g.R * g.wr + words - 1) / words; }
 
@@ -479,7 +479,8 @@ void launch_field_adjoint(const Grid& g, const float* f, float iso, const uint32
                           const WordOffsets* o, const float* dverts, const float* dgrad,
                           float* out, int num_sms, cudaStream_t s) {
   if (dgrad) {
-    const MarchTiles mt = march_tiles_for(adj_nxw(g), adj_bands(g), g.nz, adjoint_wave(num_sms));
+    const MarchBox box = adjoint_box(g);
+    const MarchTiles mt = adj_tiles(g, march_seg(&box, 1, adjoint_wave(num_sms), kAdjSeg));
     k_grad_adjoint<<<(unsigned)mt.tasks, 32, kAdjSmem, s>>>(g, dgrad, out, mt);
   } else {
     cudaMemsetAsync(out, 0, (size_t)g.P * sizeof(float), s);

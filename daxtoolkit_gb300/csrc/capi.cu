@@ -1184,7 +1184,8 @@ int dax_gb300_mc_batch_create(int num_grids, const dax_gb300_uniform_grid* grids
     large += daxgb::adjoint_edge_blocks(g, daxgb::kEdgeWordsMost);
   }
   b->grad_seg = daxgb::march_seg(gbox.data(), num_grids, daxgb::grad_wave(num_sms()), daxgb::kGradSeg);
-  b->adj_seg = daxgb::march_seg(abox.data(), num_grids, daxgb::adjoint_wave(num_sms()), daxgb::kSeg);
+  b->adj_seg = daxgb::march_seg(abox.data(), num_grids, daxgb::adjoint_wave(num_sms()),
+                                daxgb::kAdjSeg);
   // two waves of the larger blocks, four an SM, or more
   b->edge_words = large >= 8ll * num_sms() ? daxgb::kEdgeWordsMost : daxgb::kEdgeWordsLeast;
   for (int i = 0; i < num_grids; ++i) {

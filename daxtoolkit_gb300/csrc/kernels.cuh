@@ -251,7 +251,12 @@ void launch_thr_emit(const Grid& g, const float* f, const WordOffsets& o, const 
 // marched along z; an adjoint block is one warp.  Band heights and register
 // budgets (blocks per SM) were chosen by timing on GB300.
 constexpr int kMarchCols = 31;
-constexpr int kSeg = 32;            // planes a segment of a grid set's adjoint tiles, at most
+// Planes per adjoint tile, at most.  A tile takes its planes one after another
+// and reads one plane for nothing, but tiles that start together do not end
+// together, and short ones level that out: 385 x 321 x 289 128 us in one wave of
+// 42 planes, 115, 109, 105, 103 and 105 with 21, 10, 6, 5 and 4; 257 x 301 x 333
+// 97 with 28, 81 with 4 to 6, 95 with 2; 512^3 388 and 339 with 16 and 6.
+constexpr int kAdjSeg = 6;
 constexpr int kGradBand = 4;        // cell rows per CellGradient tile
 constexpr int kGradSeg = 16;        // cell planes per CellGradient tile, at most
 constexpr int kGradWarps = 4;       // CellGradient tiles (warps) per block
@@ -295,26 +300,6 @@ inline int march_seg(const MarchBox* box, int count, long long wave, int most) {
     if (n <= wave) return seg;
   }
   return most;
-}
-
-// The number of segments that wastes least of one grid's adjoint: a wave of
-// `wave` resident tiles runs as long as a segment, which also reads one halo
-// plane and takes about a plane's time to start.  (Cutting the planes of all
-// tiles into equal runs, so that one wave ends together, left neighbouring
-// tiles in different planes and read shared lines twice: 1.5 times the DRAM
-// traffic, 123 -> 162 us at 385 x 321 x 289.)
-inline MarchTiles march_tiles_for(int nxw, int nband, int planes, long long wave) {
-  MarchTiles best{};
-  long long least = -1;
-  for (int nseg = (planes + 63) / 64; nseg <= (planes + kLeastSeg - 1) / kLeastSeg; ++nseg) {
-    const MarchTiles mt = march_tiles(nxw, nband, planes, nseg);
-    const long long cost = (mt.tasks + wave - 1) / wave * (mt.seg + 2);
-    if (least < 0 || cost < least) {
-      least = cost;
-      best = mt;
-    }
-  }
-  return best;
 }
 
 // dL/dfield from dL/d(merged vertices) (needs the count pass's bits and
