@@ -110,27 +110,34 @@ __device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_warp, uns
 // Warp w of a tile takes the kMtChunk consecutive cells of chunk 8 * tile + w;
 // the chunk's and the tile's triangle totals are stored.
 //
-// Bound by the connectivity's bytes (16 a cell): 83 million cells take 226 us,
-// 1.44 GB at 6.4 TB/s.  A bulk copy brings the ids of kMtGroup cells into the
+// Bound by the connectivity's bytes (16 a cell): 83 million cells take 222 us,
+// 1.44 GB at 6.5 TB/s.  A bulk copy brings the ids of kMtGroup cells into the
 // warp's buffer, and as soon as they are in registers the next group's is issued,
 // also over the end of a tile.  A lane takes kMtRun consecutive cells: in a mesh of
 // tetrahedralized voxels, five cells each, the lanes then gather the same corner
 // of consecutive voxels, one or two lines a load.  The twenty ids of a lane are
-// checked by one unsigned maximum and their gathers issued together; a warp whose
-// cells reach past the end or list a bad id goes cell by cell.
+// checked by one unsigned maximum and their gathers issued together; a group that
+// reaches past the end or lists a bad id goes cell by cell.
 //
-// If the lanes' runs lie apart, more than half of them over 32 ids from the run
-// before, the lanes take consecutive cells instead, which then share lines within
-// a voxel: 471 us for voxels in random order, 683 by runs.
+// If the lanes' runs lie apart, more than half of them over 32 ids from the run of
+// two lanes before (neighbouring voxels list their corners in other orders), a
+// lane takes one corner of eight cells instead: L1 looks up a line at a time, and
+// the corners of a cell, asked for together, share lines where the points are in
+// order, whatever the order of the cells.  A vote on the values is then eight
+// cells' cases.  (A corner of 32 cells a load took 1240 us, count and scan, for
+// cells in no order, now 995; voxels in random order 478 and 427.)
 //
-// (A cell a lane, with loads straight from global memory, touched 4 to 8 lines a
-// gather, which L1 looks up one at a time: 276 us, and 543 for voxels in random
-// order.  Runs with a check a cell were issue bound, 81 instructions a row of 32
-// cells: 292.  Two buffers a warp took as long, but left the gathers half the L1:
-// 2040 us for cells in no order at all, now 1280; the one order for which a cell a
-// lane was faster, 1080.)
+// Gathers in no order also need L1 as room for the lines on their way: the buffers
+// of four blocks are held below 100 KB.  With 132 KB, 1057 and 454 us; points in no
+// order either, 1290 and now 1203.
 //
-// Connectivity that is not 16-byte aligned is copied by plain loads: 376 us, as before.
+// (A cell a lane, with loads straight from global memory: 301 us in order, 1082 for
+// cells and 552 for voxels in random order, 1211 for cells and points in none.
+// Runs with a check a cell were issue bound, 81 instructions a row of 32 cells:
+// 292.  Two buffers a warp took as long, but left the gathers half the L1: 2040 us
+// for cells in no order.)
+//
+// Connectivity that is not 16-byte aligned is copied by plain loads: 387 us.
 constexpr int kMtRun = 5;
 constexpr int kMtGroup = 32 * kMtRun;
 constexpr int kMtGroups = kMtChunk / kMtGroup;  // whole groups a chunk; the rest a cell a lane
@@ -145,7 +152,7 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
   constexpr int kWarps = kMtThreads / 32;
   __shared__ unsigned s_warp[2][kWarps];
   __shared__ __align__(16) int4 s_ids[kWarps][kMtGroup];
-  __shared__ __align__(16) uint8_t s_case[kWarps][kMtChunk];
+  __shared__ __align__(16) uint8_t s_case[kWarps][kMtGroups * kMtGroup];
   __shared__ uint64_t s_bar[kWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint8_t* const cs_of = s_case[wid];
@@ -193,10 +200,11 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
     }
     __syncwarp();
   };
-  auto classify = [&](const int4& q) -> int {
+  // a cell whose ids need not be points
+  auto classify = [&](const int4& q, bool& is) -> int {
     const bool ok = q.x >= 0 && (long long)q.x < P && q.y >= 0 && (long long)q.y < P && q.z >= 0 &&
                     (long long)q.z < P && q.w >= 0 && (long long)q.w < P;
-    bad = bad || !ok;
+    is = is && ok;
     if (!ok) return 0;
     const float v[4] = {__ldg(f + q.x), __ldg(f + q.y), __ldg(f + q.z), __ldg(f + q.w)};
     return mt_classify(v, iso);
@@ -212,52 +220,73 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
       landed(g);
       if (late) break;
       const int4* ids = s_ids[wid];
+      uint8_t* const out = cs_of + g * kMtGroup;
+      const long long cg = cb + g * kMtGroup;
       int4 q[kMtRun];
-      int first = kMtRun * lane, step = 1;  // the lane's cells of the group
-      q[0] = ids[first];
-      const int before = __shfl_up_sync(kFull, q[0].x, 1);
-      if (__popc(__ballot_sync(kFull, (unsigned)(q[0].x - before + 32) > 64u)) > 16) {
-        first = lane;
-        step = 32;
-        q[0] = ids[first];
-      }
-      unsigned top = max(max((unsigned)q[0].x, (unsigned)q[0].y),
-                         max((unsigned)q[0].z, (unsigned)q[0].w));
+      q[0] = ids[kMtRun * lane];
+      const int before = __shfl_up_sync(kFull, q[0].x, 2);
+      const bool apart =
+          __popc(__ballot_sync(kFull, (unsigned)q[0].x - (unsigned)before + 32u > 64u)) > 16;
+      if (apart) {
 #pragma unroll
-      for (int i = 1; i < kMtRun; ++i) {
-        q[i] = ids[first + i * step];
-        top = max(max(top, max((unsigned)q[i].x, (unsigned)q[i].y)),
-                  max((unsigned)q[i].z, (unsigned)q[i].w));
+        for (int i = 0; i < kMtRun; ++i) {
+          const int* const w = reinterpret_cast<const int*>(ids) + 128 * i + lane;
+          q[i] = make_int4(w[0], w[32], w[64], w[96]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 1; i < kMtRun; ++i) q[i] = ids[kMtRun * lane + i];
       }
-      const int at = g * kMtGroup + first;
-      // Whether every lane's ids are points.  The vote takes each lane's loaded
+      unsigned top = 0;
+#pragma unroll
+      for (int i = 0; i < kMtRun; ++i)
+        top = max(top, max(max((unsigned)q[i].x, (unsigned)q[i].y),
+                           max((unsigned)q[i].z, (unsigned)q[i].w)));
+      // Whether every id is a point of the mesh.  The vote takes each lane's loaded
       // values, so all of the loads have returned before the buffer is filled
       // again (a barrier alone lets the copy pass loads that still wait); the fence
       // orders them before the copy's writes.
-      const bool fast = __all_sync(kFull, top < points && cb + at + (kMtRun - 1) * step < C);
+      const bool fast = __all_sync(kFull, top < points && cg + kMtGroup <= C);
+      if (!fast) {
+        bool is = true;
+#pragma unroll 1
+        for (int i = lane; i < kMtGroup; i += 32) {
+          const int cs = cg + i < C ? classify(ids[i], is) : 0;
+          out[i] = (uint8_t)cs;
+          sum += (unsigned)mt_faces(cs);
+        }
+        bad = __any_sync(kFull, !is) || bad;  // as above, every load has returned
+      }
       if (VEC) fence_proxy_async();
       __syncwarp();
       copy(tile, g + 1);
-      if (fast) {
-        float v[kMtRun][4];
+      if (!fast) continue;
+      float v[kMtRun][4];
+#pragma unroll
+      for (int i = 0; i < kMtRun; ++i) {
+        v[i][0] = __ldg(f + q[i].x);
+        v[i][1] = __ldg(f + q[i].y);
+        v[i][2] = __ldg(f + q[i].z);
+        v[i][3] = __ldg(f + q[i].w);
+      }
+      if (apart) {
+        // a vote is eight cells' cases: cell 32 i + lane is the lane's four bits of
+        // vote lane / 8
 #pragma unroll
         for (int i = 0; i < kMtRun; ++i) {
-          v[i][0] = __ldg(f + q[i].x);
-          v[i][1] = __ldg(f + q[i].y);
-          v[i][2] = __ldg(f + q[i].z);
-          v[i][3] = __ldg(f + q[i].w);
-        }
+          unsigned b[4];
 #pragma unroll
-        for (int i = 0; i < kMtRun; ++i) {
-          const int cs = mt_classify(v[i], iso);
-          cs_of[at + i * step] = (uint8_t)cs;
+          for (int n = 0; n < 4; ++n) b[n] = __ballot_sync(kFull, v[i][n] > iso);
+          const unsigned lo = lane & 8 ? b[1] : b[0], hi = lane & 8 ? b[3] : b[2];
+          const int cs = (int)((lane & 16 ? hi : lo) >> (4 * (lane & 7)) & 15u);
+          out[32 * i + lane] = (uint8_t)cs;
           sum += (unsigned)mt_faces(cs);
         }
       } else {
 #pragma unroll
         for (int i = 0; i < kMtRun; ++i) {
-          const int cs = cb + at + i * step < C ? classify(q[i]) : 0;
-          cs_of[at + i * step] = (uint8_t)cs;
+          const int cs = mt_classify(v[i], iso);
+          out[kMtRun * lane + i] = (uint8_t)cs;
           sum += (unsigned)mt_faces(cs);
         }
       }
@@ -278,15 +307,17 @@ __global__ void __launch_bounds__(kMtThreads, VEC ? 4 : 5)
         const float v[4] = {__ldg(f + q.x), __ldg(f + q.y), __ldg(f + q.z), __ldg(f + q.w)};
         cs = mt_classify(v, iso);
       }
-      cs_of[at] = (uint8_t)cs;
+      if (cb + at < C) cases[cb + at] = (uint8_t)cs;
       sum += (unsigned)mt_faces(cs);
     }
     __syncwarp();
     // the chunk's cases in whole lines
-    if (cb + kMtChunk <= C && (reinterpret_cast<uintptr_t>(cases) & 15) == 0) {
-      reinterpret_cast<uint4*>(cases + cb)[lane] = reinterpret_cast<const uint4*>(cs_of)[lane];
+    constexpr int kStaged = kMtGroups * kMtGroup;
+    if (cb + kStaged <= C && (reinterpret_cast<uintptr_t>(cases) & 15) == 0) {
+      if (lane < kStaged / 16)
+        reinterpret_cast<uint4*>(cases + cb)[lane] = reinterpret_cast<const uint4*>(cs_of)[lane];
     } else {
-      for (int i = lane; i < kMtChunk && cb + i < C; i += 32) cases[cb + i] = cs_of[i];
+      for (int i = lane; i < kStaged && cb + i < C; i += 32) cases[cb + i] = cs_of[i];
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFull, sum, d);
@@ -963,6 +994,15 @@ void launch_mt_count(const int32_t* conn, long long C, const float* f, long long
   unsigned* tot = reinterpret_cast<unsigned*>(scratch + L.tile_tot);
   unsigned* ctot = reinterpret_cast<unsigned*>(scratch + L.chunk_tot);
   if (vec) {
+    // four blocks in 100 KB of shared memory, so that L1 keeps 156 KB (a hint; set
+    // once per device): left to itself the driver takes 132 KB
+    static int hinted[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !hinted[dev]) {
+      cudaFuncSetAttribute(k_mt_count<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 43);
+      hinted[dev] = 1;
+    }
     const int b = resident_blocks(k_mt_count<true>, kMtThreads, 0, num_sms, L.tiles);
     k_mt_count<true><<<b, kMtThreads, 0, s>>>(conn, C, f, P, iso, cases, tot, ctot, info, L.tiles,
                                               polls);
