@@ -28,10 +28,10 @@ __device__ __forceinline__ float magsq3(float x, float y, float z) {
 
 // worklet::Mandlebulb (Benchmarks/Mandlebulb/Worklets.h:65-109): the escape
 // iteration of pos -> pos^10 + c (White and Nylander's power, :92-108), 0
-// when c itself is outside radius sqrt(2), at most 35.  One step of it.
-__device__ __forceinline__ void mandelbulb_step(float& x, float& y, float& z, float cx, float cy,
-                                                float cz) {
-  const float r2 = magsq3(x, y, z);
+// when c itself is outside radius sqrt(2), at most 35.
+// One step of it; r2 is the point's squared radius, before and after.
+__device__ __forceinline__ void mandelbulb_step(float& x, float& y, float& z, float& r2, float cx,
+                                                float cy, float cz) {
   const float t = __fsqrt_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)));
   const float thetaN = __fmul_rn(10.0f, atan2f(t, z));
   const float phiN = __fmul_rn(10.0f, atan2f(y, z));
@@ -44,58 +44,71 @@ __device__ __forceinline__ void mandelbulb_step(float& x, float& y, float& z, fl
   x = __fadd_rn(px, cx);
   y = __fadd_rn(py, cy);
   z = __fadd_rn(pz, cz);
+  r2 = magsq3(x, y, z);
 }
 
 // Bound by arithmetic: two arctangents, a power, a sine and cosine, a tangent
 // and a sine a step, 1 to 34 steps a point.  With a point per lane a warp
 // steps until its slowest lane is done, so a lane that is done takes the
 // block's next point instead (its tiles of 256 points, strided by the grid,
-// in order, from a counter in shared memory), once kRefill lanes wait.
-constexpr int kRefill = 4;
+// in order, from a counter in shared memory), once kRefill lanes wait: the 201^3
+// points of [-1, 1]^3 945 us with a point per lane, 757 so; 49^3 41 and 43.  Where
+// all points of a warp take the same steps it only costs, a refill about 45
+// instructions more than a loop over points: 201^3 points inside the fractal, 34
+// steps each, 2030 and 2132, one step each 86 and 98, none (radius above sqrt(2))
+// 27 and 36.  (2, 4 and 8 lanes: 783, 761 and 758.  Testing for a refill after
+// every step, in the same loop: 787, and 2235 inside.  Stepping the waiting lanes
+// too, without a branch: 829.)
+constexpr int kRefill = 6;
 
-__global__ void __launch_bounds__(256) k_mandelbulb_field(Grid g, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_mandelbulb_field(Grid g, unsigned long long mnx,
+                                                          float* __restrict__ out) {
   __shared__ unsigned s_next;
   if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
   const unsigned P = (unsigned)g.P, tiles = (P + 255u) / 256u;
-  const unsigned mine = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 256u;  // points, past P too
-  float x = 0, y = 0, z = 0, cx = 0, cy = 0, cz = 0;
+  // the block's points; the last tile is the last one of its block
+  const unsigned mine = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x * 256u -
+                        ((tiles - 1u) % gridDim.x == blockIdx.x ? tiles * 256u - P : 0u);
+  float x = 0, y = 0, z = 0, r2 = 0, cx = 0, cy = 0, cz = 0;
   unsigned p = 0;
   int i = 0;  // the step the lane is at; 0: it has no point
+  unsigned idle = kFull;
   bool more = true;
   while (true) {
-    const unsigned idle = __ballot_sync(kFull, i == 0);
-    if (more && __popc(idle) >= kRefill) {
+    if (more) {
       unsigned n = 0;
-      if (lane == 0) n = atomicAdd(&s_next, (unsigned)__popc(idle));
+      if (below == 0u) n = atomicAdd(&s_next, (unsigned)__popc(idle));
       n = __shfl_sync(kFull, n, 0);
       more = n + (unsigned)__popc(idle) < mine;
-      n += (unsigned)__popc(idle & ((1u << lane) - 1u));
-      p = i == 0 ? ((n >> 8) * gridDim.x + blockIdx.x) * 256u + (n & 255u) : p;
-      if (i == 0 && n < mine && p < P) {
-        const unsigned row = p / (unsigned)g.nx;
+      n += (unsigned)__popc(idle & below);
+      if (i == 0 && n < mine) {
+        p = (n >> 8) * (256u * gridDim.x) + 256u * blockIdx.x + (n & 255u);
+        const unsigned row = div_by(p, mnx);
         int j, k;
         split_row(g, row, j, k);
         x = cx = coord(g.ox, g.sx, (int)(p - row * (unsigned)g.nx), g.mx);
         y = cy = coord(g.oy, g.sy, j, g.my);
         z = cz = coord(g.oz, g.sz, k, g.mz);
-        if (magsq3(x, y, z) > 2.0f) out[p] = 0.0f;
+        r2 = magsq3(x, y, z);
+        if (r2 > 2.0f) out[p] = 0.0f;
         else i = 1;
       }
-    } else if (idle == kFull) {
-      break;
+      idle = __ballot_sync(kFull, i == 0);
     }
-    if (i > 0) {
-      mandelbulb_step(x, y, z, cx, cy, cz);
-      const bool escaped = magsq3(x, y, z) > 2.0f;
-      if (escaped || i == 34) {
-        out[p] = escaped ? (float)i : 35.0f;
-        i = 0;
-      } else {
-        ++i;
+    // steps until kRefill lanes wait or, with no points left, until all do
+    const int most = more ? kRefill : 32;
+    while (__popc(idle) < most) {
+      if (i > 0) {
+        mandelbulb_step(x, y, z, r2, cx, cy, cz);
+        const bool escaped = r2 > 2.0f;
+        if (escaped || i == 34) out[p] = escaped ? (float)i : 35.0f;
+        i = escaped || i == 34 ? 0 : i + 1;
       }
+      idle = __ballot_sync(kFull, i == 0);
     }
+    if (!more && idle == kFull) break;
   }
 }
 
@@ -175,7 +188,7 @@ __global__ void __launch_bounds__(256) k_colors_and_norms(const float* __restric
 
 void launch_mandelbulb_field(const Grid& g, float* out, int num_sms, cudaStream_t s) {
   const int b = resident_blocks(k_mandelbulb_field, 256, 0, num_sms, (g.P + 255) / 256);
-  k_mandelbulb_field<<<b, 256, 0, s>>>(g, out);
+  k_mandelbulb_field<<<b, 256, 0, s>>>(g, div_multiplier((unsigned)g.nx), out);
 }
 
 void launch_colors_and_norms(const float* verts, long long nv, float* norms, uint8_t* colors,
