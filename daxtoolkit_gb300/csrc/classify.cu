@@ -39,7 +39,7 @@ __device__ __forceinline__ T ld_field(const T* p, bool keep) {
 }
 
 template <int MODE, bool VEC, bool KEEP>
-__global__ void __launch_bounds__(256, 5) k_classify_bits(GridSet S, uint32_t* __restrict__ bits,
+__global__ void __launch_bounds__(256) k_classify_bits(GridSet S, uint32_t* __restrict__ bits,
                                                        long long nwords, long long c_begin,
                                                        long long c_end, Info* init) {
   constexpr int UNROLL = 4;
