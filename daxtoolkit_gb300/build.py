@@ -8,6 +8,7 @@ nothing but the driver.  No fast-math: the kernels spell out every rounding
 (``__fmul_rn``/``__fadd_rn``/``__fdiv_rn``) to match the reference's float
 arithmetic bit for bit.
 """
+import glob
 import os
 import platform
 import shutil
@@ -24,8 +25,6 @@ LIB = os.path.join(LIBDIR, "libdax_gb300.so")
 SOURCES = ["classify.cu", "mc.cu", "pipeline.cu", "threshold.cu", "gradient.cu", "adjoint.cu", "capi.cu",
            "noalloc.cu", "memory.cu", "fused.cu", "primitives.cu", "slice.cu", "mt.cu",
            "mandelbulb.cu", "fields.cu", "vtk.cu", "selftest.cu"]
-HEADERS = ["common.cuh", "kernels.cuh", "mc_case.cuh", "mc_tables.h", "mt_tables.h",
-           "coolwarm_table.h"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
                      "-Xptxas", "-warn-spills", "--expt-relaxed-constexpr"]
@@ -44,6 +43,12 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def headers():
+    """Every header a source may include: an object older than any of them is stale."""
+    return sorted(p for d in (CSRC, os.path.join(HERE, "..", "include"))
+                  for ext in ("*.h", "*.cuh") for p in glob.glob(os.path.join(d, ext)))
+
+
 def build(force=False, verbose=False):
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(OBJDIR, exist_ok=True)
@@ -54,13 +59,12 @@ def build(force=False, verbose=False):
         force = True
         open(stamp, "w").write(arch)
     include = os.path.join(HERE, "..", "include")
-    headers = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(include, "dax_gb300.h")]
     objs, jobs = [], []
     for src in SOURCES:
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJDIR, src.replace(".cu", ".o"))
         objs.append(o)
-        if force or _stale(o, [s] + headers):
+        if force or _stale(o, [s] + headers()):
             jobs.append([nvcc()] + NVCC_FLAGS + ["-I", include, "-c", s, "-o", o])
 
     def run(cmd):
