@@ -35,11 +35,16 @@ def _ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
 
+# The current stream's raw handle, where torch has it: building torch's Stream
+# object took 3 of the 54 us of a call on a small grid.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream=None):
-    if stream is not None:
-        return ctypes.c_void_p(stream.cuda_stream)
-    # the raw handle: building torch's Stream object took 3 of the 54 us of a call on a small grid
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    if stream is None and _raw_stream is not None:
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+    s = stream if stream is not None else torch.cuda.current_stream()
+    return ctypes.c_void_p(s.cuda_stream)
 
 
 def _require_field(field, grid):
