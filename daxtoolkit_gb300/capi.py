@@ -142,6 +142,7 @@ SIGNATURES = {
                                       ctypes.c_uint32, vp, vp], i32),
     "dax_gb300_selfcheck_mt_wait": ([vp, i64, vp, i64, f32, vp, sz, vp], i32),
     "dax_gb300_selfcheck_scan_wait": ([vp, vp, i64, ctypes.c_uint32, i32, vp, sz, vp, vp], i32),
+    "dax_gb300_selfcheck_sort_wait": ([vp, vp, i64, ctypes.c_uint32, vp, sz, vp], i32),
     "dax_gb300_scan_scratch_bytes": ([i64], sz),
     "dax_gb300_scan": ([vp, vp, i64, i32, i32, vp, sz, vp, vp], i32),
     "dax_gb300_sort_scratch_bytes": ([i64, i32, i32], sz),

@@ -993,10 +993,10 @@ constexpr int kLook = 4;
 template <typename U>
 __device__ __forceinline__ uint32_t digit_look_back(const uint32_t* state, int tile, unsigned d,
                                                     const U* kin, long long n, int shift,
-                                                    const KeyOrder<U>& ord) {
+                                                    const KeyOrder<U>& ord, unsigned polls) {
   uint32_t prefix = 0;
   int t = tile - 1;
-  Spin spin;
+  Spin spin(polls);
   while (t >= 0) {
     uint32_t v[kLook];
 #pragma unroll
@@ -1038,8 +1038,9 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
                                            uint32_t* __restrict__ vout, long long n, int shift,
                                            const uint32_t* __restrict__ hist,
                                            uint32_t* __restrict__ state, int tile,
-                                           const KeyOrder<U>& ord, U* s_key, uint32_t* s_val,
-                                           uint32_t* s_cnt, uint32_t* s_dst, uint32_t* s_warp) {
+                                           const KeyOrder<U>& ord, unsigned polls, U* s_key,
+                                           uint32_t* s_val, uint32_t* s_cnt, uint32_t* s_dst,
+                                           uint32_t* s_warp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long tb = (long long)tile * kSweepTile;
   const int valid = FULL ? kSweepTile : (int)(n - tb);
@@ -1093,7 +1094,8 @@ __device__ __forceinline__ void sweep_tile(const U* __restrict__ kin, U* __restr
     asm volatile("bar.sync 1, 256;" ::: "memory");  // the 256 digit threads
     x -= h;
     for (int w = 0; w < warp; ++w) x += s_warp[8 + w];
-    const uint32_t before = digit_look_back(state, tile, (unsigned)tid, kin, n, shift, ord);
+    const uint32_t before = digit_look_back(state, tile, (unsigned)tid, kin, n, shift, ord,
+                                            polls);
     if (tile > 0) st_relaxed(mine, kSortInc | (before + tot));
     s_dst[tid] = x + before - lstart;
   }
@@ -1134,7 +1136,7 @@ __global__ void __launch_bounds__(kSweepThreads, (kSweepBlocks<U, VW>))
     k_radix_sweep(const U* __restrict__ kin, U* __restrict__ kout, const uint32_t* __restrict__ vin,
                   uint32_t* __restrict__ vout, long long n, int shift,
                   const uint32_t* __restrict__ hist, uint32_t* __restrict__ state,
-                  unsigned* __restrict__ ticket, KeyOrder<U> ord) {
+                  unsigned* __restrict__ ticket, KeyOrder<U> ord, unsigned polls) {
   extern __shared__ unsigned long long s_dyn[];
   U* s_key = reinterpret_cast<U*>(s_dyn);                            // [kSweepTile]
   uint32_t* s_val = reinterpret_cast<uint32_t*>(s_key + kSweepTile);  // [kSweepTile] if VW
@@ -1148,11 +1150,11 @@ __global__ void __launch_bounds__(kSweepThreads, (kSweepBlocks<U, VW>))
   const int tile = s_tile;
   if ((long long)tile * kSweepTile >= n) return;
   if ((long long)(tile + 1) * kSweepTile <= n)
-    sweep_tile<U, VW, true>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, s_key, s_val,
-                            s_cnt, s_dst, s_warp);
+    sweep_tile<U, VW, true>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, polls, s_key,
+                            s_val, s_cnt, s_dst, s_warp);
   else
-    sweep_tile<U, VW, false>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, s_key, s_val,
-                             s_cnt, s_dst, s_warp);
+    sweep_tile<U, VW, false>(kin, kout, vin, vout, n, shift, hist, state, tile, ord, polls, s_key,
+                             s_val, s_cnt, s_dst, s_warp);
 }
 
 // At most kSortTile elements: every pass in one block's shared memory, the
@@ -1487,17 +1489,17 @@ SortLayout sort_layout(long long n, int key_bytes, int value_bytes) {
 template <typename U, int VW>
 void launch_sweep(const U* kin, U* kout, const uint32_t* vin, uint32_t* vout, long long n, int shift,
                   const uint32_t* hist, uint32_t* state, unsigned* ticket, KeyOrder<U> ord,
-                  cudaStream_t s) {
+                  unsigned polls, cudaStream_t s) {
   static int opted[64] = {};
   constexpr size_t smem = sweep_smem<U>(VW);
   opt_in_smem((const void*)k_radix_sweep<U, VW>, smem, opted);
   k_radix_sweep<U, VW><<<sort_tiles(n), kSweepThreads, smem, s>>>(kin, kout, vin, vout, n, shift,
-                                                                hist, state, ticket, ord);
+                                                                hist, state, ticket, ord, polls);
 }
 
 // passes: 8-bit digits to sort, least significant first (an even count, so
 // the result ends in keys/vals); plain = the keys are unsigned, ascending and
-// need no order mapping.
+// need no order mapping; polls: the most polls of a look-back's wait.
 //
 // Up to kSortTile elements are one launch of one block.  Longer arrays keep
 // the tile states, the digit counts and the tickets in the scratch's
@@ -1507,7 +1509,7 @@ void launch_sweep(const U* kin, U* kout, const uint32_t* vin, uint32_t* vout, lo
 template <typename U>
 void radix_sort(U* keys, uint32_t* vals, int vwords, long long n, int kind, bool desc,
                 char* scratch, int num_sms, cudaStream_t s, int passes = (int)sizeof(U),
-                bool plain = false) {
+                bool plain = false, unsigned polls = kSpinIters) {
   if (n <= kSortTile) {
     static int opted[64] = {};
     const KeyOrder<U> ord{kind, desc, !plain, !plain};
@@ -1541,11 +1543,11 @@ void radix_sort(U* keys, uint32_t* vals, int vwords, long long n, int kind, bool
     if (at == 0) k_radix_hist<U><<<bh, kSortThreads, 0, s>>>(ksrc, n, p, counted, hist, ord);
     const uint32_t* h = hist + 256 * at;
     switch (vwords) {
-      case 0: launch_sweep<U, 0>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
-      case 1: launch_sweep<U, 1>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
-      case 2: launch_sweep<U, 2>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
-      case 3: launch_sweep<U, 3>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
-      default: launch_sweep<U, 4>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, s); break;
+      case 0: launch_sweep<U, 0>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, polls, s); break;
+      case 1: launch_sweep<U, 1>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, polls, s); break;
+      case 2: launch_sweep<U, 2>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, polls, s); break;
+      case 3: launch_sweep<U, 3>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, polls, s); break;
+      default: launch_sweep<U, 4>(ksrc, kdst, vsrc, vdst, n, 8 * p, h, state, ticket, ord, polls, s); break;
     }
   }
 }
@@ -1759,6 +1761,19 @@ int dax_gb300_sort_by_key(void* d_keys, void* d_values, int64_t n, int key_type,
     radix_sort<unsigned long long>(static_cast<unsigned long long*>(d_keys),
                                    static_cast<uint32_t*>(d_values), value_bytes / 4, n, kind,
                                    descending != 0, sc, prim_sms(), s);
+  return launched("sort kernels");
+}
+
+int dax_gb300_selfcheck_sort_wait(uint32_t* d_keys, uint32_t* d_values, int64_t n, uint32_t polls,
+                                  void* d_scratch, size_t scratch_bytes, void* stream) {
+  using namespace daxgb;
+  if (!size_ok(n) || n <= kSortTile) return bad("the sort must be of more than one block");
+  if (!d_keys || !d_values || !d_scratch) return bad("NULL keys, values or scratch");
+  if (scratch_bytes < dax_gb300_sort_scratch_bytes(n, DAX_GB300_TYPE_U32, 4))
+    return bad("scratch smaller than dax_gb300_sort_scratch_bytes()");
+  radix_sort<uint32_t>(d_keys, d_values, 1, n, 0, false, static_cast<char*>(d_scratch), prim_sms(),
+                       static_cast<cudaStream_t>(stream), 4, false,
+                       polls < kSpinIters ? polls : kSpinIters);
   return launched("sort kernels");
 }
 

@@ -143,6 +143,13 @@ int dax_gb300_selfcheck_mt_wait(const int32_t* d_conn, int64_t num_cells, const 
 int dax_gb300_selfcheck_scan_wait(const int32_t* d_in, int32_t* d_out, int64_t n, uint32_t polls,
                                   int lost, void* d_scratch, size_t scratch_bytes, int32_t* h_total,
                                   void* stream);
+
+/* Self-check of the radix sort's bounded waits: more than 8192 uint32 keys,
+ * ascending, with a 32-bit value each, whose waits for earlier tiles' digit
+ * counts run out after `polls` polls.  A count that did not come is taken from
+ * the keys, so the result is the same. */
+int dax_gb300_selfcheck_sort_wait(uint32_t* d_keys, uint32_t* d_values, int64_t n, uint32_t polls,
+                                  void* d_scratch, size_t scratch_bytes, void* stream);
 const char* dax_gb300_last_error(void);
 
 /* Sets the message dax_gb300_last_error() returns on this thread and returns
