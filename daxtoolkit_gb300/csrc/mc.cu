@@ -725,14 +725,16 @@ __device__ __forceinline__ void cell_edge_ids(const uint32_t* st, int s, int q, 
 }
 
 // A warp takes up to `batch` (1..32) active words at a time from the counter
-// *ticket; the last block to finish resets *ticket and *done.  While there is
-// more than one round of them left, a batch is half of a warp's share of what
-// is left, so that the rounds shrink and the warps end together; then it is the
-// share, down to kEmitLeast words.  (Merged, a round of up to 20 words a warp
-// costs less than two smaller ones: 19 against 23 us on a slice of 383 x 405 x
-// 331.  Unmerged, words differ more and the line lies at 6: 79 against 100 us
-// on the Mandelbulb.  Fixed batches of 16: 24 -> 14 us for the 128^3 benchmark,
-// 27 -> 20 for 301 x 257 x 199, 45 -> 43 at 512^3.)
+// *ticket; the last block to finish resets *ticket and *done.  Merged, a batch is
+// at most a warp's share of what is left, down to kEmitLeast words: 17 -> 13 us for
+// 128^3 blobs, 24 -> 22 at 300^3, 42 -> 41 at 512^3 against fixed batches of 16.
+// (Halving it while there is more than one round left, so that the rounds shrink
+// and the warps end together, costs more than it levels out: with the line at 20
+// words a warp 83 us in place of 68 for 64^3 points of noise, 24.5 in place of
+// 21.7 on a slice of 400^3.)  Unmerged, where words differ more, it is half the
+// share above 6 words a warp: 34 -> 19 us for 128^3 blobs, 85 -> 69 at 512^3; with
+// the line at 3, 6, 10 and 20, 31, 31, 35 and 42 us at 300^3, 83, 83, 86 and 100 on
+// the 201^3 Mandelbulb.
 //
 // Unmerged, the vertices of a chunk of 32 cells are dealt to the lanes in
 // output order: a lane looping over its own cell's triangles kept 16 of 32
@@ -803,7 +805,8 @@ __global__ void __launch_bounds__(kEmitWarps * 32, 4) k_mc_emit(GridSet S,
     // the next batch of active words, taken dynamically (batches differ
     // widely in cost); its size from what was left at the last one
     const long long each = (left + warps - 1) / warps;
-    const int take = (int)min((long long)batch, each > (MERGE ? 20 : 6) ? each / 2 : max(each, (long long)kEmitLeast));
+    const long long share = !MERGE && each > 6 ? each / 2 : max(each, (long long)kEmitLeast);
+    const int take = (int)min((long long)batch, share);
     long long a0 = 0;
     if (lane == 0) a0 = A0 + (long long)atomicAdd(ticket, (unsigned)take);
     a0 = __shfl_sync(kFull, a0, 0);
