@@ -887,7 +887,7 @@ class MarchingCubesBatch:
 
     def autotune(self, verts, conn, merge=True, stream=None):
         """dax_gb300_mc_batch_autotune on these outputs: keeps the fastest
-        emit batch / count pass in the plan; returns (emit_batch, dealt,
+        emit batch in the plan; returns (emit_batch, dealt as set,
         best_ms), best_ms -1 when the extent class was tuned before."""
         ms = ctypes.c_float()
         capi.call("dax_gb300_mc_batch_autotune", self.handle, int(bool(merge)), _ptr(self.scratch),

@@ -316,7 +316,7 @@ struct dax_gb300_mc_batch {
   // tuned by dax_gb300_mc_batch_autotune (or set): active words per emit
   // warp batch
   int emit_batch = daxgb::kEmitBatch;
-  int dealt = 1;  // kept for get_config: there is one count pass
+  int dealt = 1;  // set_config's, for get_config: there is one count pass
   // grid-set CellGradient and adjoint: totals of the concatenated per-cell
   // and per-point arrays, and per grid the first block of each set launch
   // (d_blk: [gradient][adjoint gradient term][adjoint vertex term], count + 1

@@ -75,7 +75,7 @@ struct GridSlot {
 
 // A set of grids processed by one launch per pass.  count == 1: the grid is
 // `one` (no table lookups); count > 1: `slots` is a device table sorted by
-// chunk0 / row0 and rows / chunks are resolved by binary search.
+// chunk0 / rw0, in which chunks and row words are found by binary search.
 struct GridSet {
   const GridSlot* slots;
   int count;
@@ -84,15 +84,6 @@ struct GridSet {
   long long rowwords;     // total row words: sum of R * wr
   GridSlot one;
 };
-
-__device__ __forceinline__ int slot_of_row(const GridSet& S, long long grow) {
-  int lo = 0, hi = S.count - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(&S.slots[mid].row0) <= grow) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
 
 __device__ __forceinline__ int slot_of_chunk(const GridSet& S, long long chunk) {
   int lo = 0, hi = S.count - 1;
@@ -172,7 +163,7 @@ struct Info {
   long long total_b;      // merged vertices (MC) / used points (threshold)
   long long total_c;      // active row words
   int error;              // kErr* bits raised on the device
-  unsigned ticket;        // next batch of active words for the MC emit warps
+  unsigned ticket;        // active words the MC emit warps have taken
   unsigned done;          // MC emit blocks finished (the last resets both)
   int pad[7];
 };
@@ -182,7 +173,7 @@ constexpr int kErrOverflow = 4;    // more than 2^31 - 1 triangles or vertices
 constexpr int kErrBadIndex = 8;    // a cell lists a point id outside [0, P)
 constexpr int kErrState = 16;      // a merge scratch that no merge pass of this count wrote
 constexpr int kErrBadCount = 32;   // a count array asks a cell for a triangle its case lacks
-constexpr int kErrTimeout = 64;    // a bounded device-side wait ran out (the fused count pass)
+constexpr int kErrTimeout = 64;    // a bounded device-side wait ran out
 
 // Coordinate of grid index i along one axis: origin + spacing * (i + min),
 // computed in float with no fused multiply-add, as the reference's implicit
@@ -304,7 +295,6 @@ __device__ __forceinline__ void row_windows4(const uint32_t* __restrict__ bits, 
   }
 }
 
-// Mask of the low n bits (n in [0, 32]).
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialization (launch_pdl) may start while the kernel before it on the
 // stream drains.  pdl_wait() blocks until that kernel has completed and its
@@ -316,6 +306,7 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Mask of the low n bits, none for n <= 0, all for n >= 32.
 __device__ __forceinline__ uint32_t low_mask(int n) {
   return n >= 32 ? kFull : (n <= 0 ? 0u : ((1u << n) - 1u));
 }

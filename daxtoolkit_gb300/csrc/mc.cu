@@ -41,37 +41,6 @@ __constant__ unsigned char kEdgeOwner[12] = {
     0 | (0 << 3), 1 | (1 << 3), 2 | (0 << 3), 0 | (1 << 3), 4 | (0 << 3), 5 | (1 << 3),
     6 | (0 << 3), 4 | (1 << 3), 0 | (2 << 3), 1 | (2 << 3), 3 | (2 << 3), 2 | (2 << 3)};
 
-// The eight corner-bit words of cells 32m..32m+31 of cell row (j, k):
-// a = (i, j, k), a1 = (i+1, j, k), b = (i, j+1, k), c = (i, j, k+1), d = (i, j+1, k+1).
-__device__ __forceinline__ CornerWords corner_words(const Grid& g, const uint32_t* bits,
-                                                   long long pos) {
-  const long long dy = g.nx, dz = (long long)g.nx * g.ny;
-  CornerWords w;
-  w.a = bits_at(bits, pos);
-  w.a1 = bits_at(bits, pos + 1);
-  w.b = bits_at(bits, pos + dy);
-  w.b1 = bits_at(bits, pos + dy + 1);
-  w.c = bits_at(bits, pos + dz);
-  w.c1 = bits_at(bits, pos + dz + 1);
-  w.d = bits_at(bits, pos + dy + dz);
-  w.d1 = bits_at(bits, pos + dy + dz + 1);
-  return w;
-}
-
-// Crossing-edge masks of point row (j, k), word m: bit q of X/Y/Z set when the
-// x/y/z edge owned by point i = 32m + q is a sign-change edge.
-__device__ __forceinline__ void crossing_masks(const Grid& g, const uint32_t* bits, int j, int k,
-                                               int m, uint32_t& X, uint32_t& Y, uint32_t& Z) {
-  const long long pos = ((long long)k * g.ny + j) * g.nx + 32ll * m;
-  const int i0 = 32 * m;
-  const uint32_t pmask = low_mask(g.nx - i0);
-  const uint32_t xmask = low_mask(g.nx - 1 - i0);
-  const uint32_t a = bits_at(bits, pos);
-  X = (a ^ bits_at(bits, pos + 1)) & xmask;
-  Y = (j < g.ny - 1) ? ((a ^ bits_at(bits, pos + g.nx)) & pmask) : 0u;
-  Z = (k < g.nz - 1) ? ((a ^ bits_at(bits, pos + (long long)g.nx * g.ny)) & pmask) : 0u;
-}
-
 // ---------------------------------------------------------------------------
 // K2: counts per row word, then the scan.
 

@@ -85,28 +85,6 @@ __device__ __forceinline__ bool load_tet(const int32_t* __restrict__ conn, long 
   return ok;
 }
 
-// Block-wide exclusive sum of small non-negative values; *total gets the sum.
-__device__ __forceinline__ unsigned block_excl(unsigned v, unsigned* s_warp, unsigned* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned x = v;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const unsigned y = __shfl_up_sync(kFull, x, d);
-    if (lane >= d) x += y;
-  }
-  if (lane == 31) s_warp[wid] = x;
-  __syncthreads();
-  unsigned before = 0, all = 0;
-  for (int w = 0; w < kMtThreads / 32; ++w) {
-    const unsigned t = s_warp[w];
-    before += w < wid ? t : 0u;
-    all += t;
-  }
-  __syncthreads();
-  *total = all;
-  return before + x - v;
-}
-
 // Warp w of a tile takes the kMtChunk consecutive cells of chunk 8 * tile + w;
 // the chunk's and the tile's triangle totals are stored.
 //
@@ -408,7 +386,8 @@ struct MtOut {
 // which with six blocks an SM gives half as many warps again: the keys of 256^3
 // points, 64 us before, take 49; the merged call went from 604 to 584 us, the
 // unmerged one from 387 to 369.
-// (Eight blocks an SM spill registers: 579 and 367.)
+// (Six spill 52 bytes in the unmerged form; eight, which spill in both, took 579
+// and 367.)
 template <bool VEC, bool KEYS>
 __global__ void __launch_bounds__(kMtThreads, 6) k_mt_emit(const float* __restrict__ pts,
                                                         const int32_t* __restrict__ conn,

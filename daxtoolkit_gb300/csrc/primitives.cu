@@ -227,8 +227,8 @@ int resident(const void* kernel, int threads, int num_sms, long long want) {
 }
 
 template <typename T>
-void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, void* d_total,
-            int num_sms, cudaStream_t s) {
+void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, int num_sms,
+            cudaStream_t s) {
   typedef typename Acc<T>::type A;
   const int tiles = ptiles(n);
   A* sums = static_cast<A*>(scratch);
@@ -236,13 +236,13 @@ void scan_t(const T* in, T* out, long long n, bool exclusive, void* scratch, voi
   k_tile_sum<T><<<b, kPT, 0, s>>>(in, n, sums, tiles);
   scan_sums<A>(sums, tiles, sums + tiles + 1, s);
   k_tile_scan<T><<<b, kPT, 0, s>>>(in, out, n, sums, tiles, exclusive ? 1 : 0);
-  if (d_total) cudaMemcpyAsync(d_total, sums + tiles, sizeof(T), cudaMemcpyDeviceToDevice, s);
 }
 
 // ---- single-pass scan of integer elements ---------------------------------
 //
-// One read and one write of every element, by one persistent block an SM.
-// A copy warp takes tiles of kSElems elements from a ticket counter and keeps
+// One read and one write of every element, by one persistent block an SM, with
+// the look-back of D. Merrill and M. Garland, "Single-pass Parallel Prefix Scan
+// with Decoupled Look-back" (NVIDIA NVR-2016-002, 2016).  A copy warp takes tiles of kSElems elements from a ticket counter and keeps
 // them in a ring of shared-memory stages (192 KB), each filled by one bulk TMA
 // copy.  Sixteen compute warps reduce a tile as soon as it lands and publish
 // its sum (AGG); a look-back warp then finds the tile's prefix over the
@@ -794,7 +794,9 @@ struct KeyOrder {
   }
 };
 
-// One sweep per digit.  A pass reads every key (and value) once and writes it
+// One sweep per digit: the method of A. Adinets and D. Merrill, "Onesweep: A
+// Faster Least Significant Digit Radix Sort for GPUs" (arXiv 2206.01784, 2022).
+// A pass reads every key (and value) once and writes it
 // once: a block takes a tile of kSweepTile elements from a ticket counter, ranks
 // its keys, publishes its count of every digit, finds how many keys of each
 // digit the earlier tiles hold by looking back over their published counts
@@ -809,7 +811,7 @@ struct KeyOrder {
 // Here equal digits are found by eight ballots, values pass through shared
 // memory like the keys, and the look-back replaces histogram and scan:
 // 0.49 ms a pass, against 0.24 ms for its 1.6 GB at the copy bandwidth.  What
-// is left is about 93 instructions a row of 32 keys and the random shared
+// is left is 108 instructions a row of 32 keys (101 M for 30 M keys) and the random shared
 // memory accesses of counters and places (63 % of that pipe), which 36 warps
 // of 16 keys a thread cannot hide from one another.  (Finding equal digits by
 // atomicOr of the lanes into a mask a digit, 16 instructions instead of 50 but
@@ -1470,8 +1472,12 @@ void compact_single(const CompactOp& op, long long n, char* scratch, int num_sms
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// keys and values of the odd passes; 1 KB per kPTile elements for digit counts
+// and tile states; the ticket.  (The scratch's size is the callers' to keep: it
+// still counts the sums of a scan of 256 counters a tile, of which the ticket
+// takes the first word.)
 struct SortLayout {
-  size_t ktmp, vtmp, hist, sums, total;
+  size_t ktmp, vtmp, hist, ticket, total;
 };
 
 SortLayout sort_layout(long long n, int key_bytes, int value_bytes) {
@@ -1481,8 +1487,8 @@ SortLayout sort_layout(long long n, int key_bytes, int value_bytes) {
   L.ktmp = 0;
   L.vtmp = align256(L.ktmp + (size_t)n * key_bytes);
   L.hist = align256(L.vtmp + (size_t)n * value_bytes);
-  L.sums = align256(L.hist + (size_t)hn * 4);
-  L.total = align256(L.sums + (size_t)sum_slots(hn) * 4);
+  L.ticket = align256(L.hist + (size_t)hn * 4);
+  L.total = align256(L.ticket + (size_t)sum_slots(hn) * 4);
   return L;
 }
 
@@ -1523,10 +1529,10 @@ void radix_sort(U* keys, uint32_t* vals, int vwords, long long n, int kind, bool
   uint32_t* vtmp = reinterpret_cast<uint32_t*>(scratch + L.vtmp);
   const int tiles = sort_tiles(n), spare = ptiles(n) - tiles;  // KB beside the states
   const int group = spare < passes ? spare : passes;           // >= 1 for n > kSortTile
-  // ... [counts of `group` passes][states][ticket], the ticket where L.sums begins
+  // ... [counts of `group` passes][states][ticket]
   uint32_t* state = reinterpret_cast<uint32_t*>(scratch + L.hist) + 256ll * spare;
   uint32_t* hist = state - 256ll * group;
-  unsigned* ticket = reinterpret_cast<unsigned*>(scratch + L.sums);
+  unsigned* ticket = reinterpret_cast<unsigned*>(scratch + L.ticket);
   const int bh = resident_blocks(k_radix_hist<U>, kSortThreads, 0, num_sms,
                                  (n + 4 * kSortThreads - 1) / (4 * kSortThreads));
   for (int p = 0; p < passes; ++p) {
@@ -1697,7 +1703,7 @@ int dax_gb300_scan(const void* d_in, void* d_out, int64_t n, int type, int exclu
   switch (type) {
     case DAX_GB300_TYPE_I32: scan_single<int32_t>((const int32_t*)d_in, (int32_t*)d_out, n, ex, sc, sms, s); break;
     case DAX_GB300_TYPE_U32: scan_single<uint32_t>((const uint32_t*)d_in, (uint32_t*)d_out, n, ex, sc, sms, s); break;
-    case DAX_GB300_TYPE_F32: scan_t<float>((const float*)d_in, (float*)d_out, n, ex, sc, nullptr, sms, s); break;
+    case DAX_GB300_TYPE_F32: scan_t<float>((const float*)d_in, (float*)d_out, n, ex, sc, sms, s); break;
     case DAX_GB300_TYPE_I64: scan_single<int64_t>((const int64_t*)d_in, (int64_t*)d_out, n, ex, sc, sms, s); break;
     default: scan_single<unsigned long long>((const unsigned long long*)d_in, (unsigned long long*)d_out, n, ex, sc, sms, s); break;
   }

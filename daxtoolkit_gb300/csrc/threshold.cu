@@ -363,8 +363,9 @@ void launch_thr_emit(const Grid& g, const float* f, const WordOffsets& o, const 
   const long long want = (g.R * g.wr + 8 * kThrBatch - 1) / (8 * kThrBatch);
   const int blocks = resident_blocks(k_thr_emit, 256, 0, num_sms, want);
   // an ordinary launch: the blocks split the active words statically, so all
-  // blocks should start together on an idle device (launched early into the
-  // SMs the scan frees, they measured 20 us slower at 512^3)
+  // blocks should start together on an idle device (count and emit, launched
+  // after and early into the SMs that the scan frees: 26.3 and 24.2 us at 100^3,
+  // 42.7 and 40.6 at 200^3, 130.7 and 130.7 at 384^3, 265.9 and 269 at 512^3)
   k_thr_emit<<<blocks, 256, 0, s>>>(g, f, kept, used, o.wt, o.wv, o.act, info, conn, kcap, coords,
                                     fout, ucap);
 }
