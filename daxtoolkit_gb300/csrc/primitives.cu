@@ -613,13 +613,17 @@ __device__ __forceinline__ void single_pass(const Op& op, long long n, int tiles
   for (int i = 0; tile[0] < tiles; ++i) {
     const int k = i % kSStages;
     tile[kAhead] = tile[kAhead - 1] < tiles ? reduce(i + kAhead, carry[kAhead]) : tiles;
-    if (!lost && !__all_sync(kFull, wait_phase(&b_pre[k], (i / kSStages) & 1, polls) && s_known[k])) {
+    // the prefix is read before the votes on it, which its loads then hide (100 M
+    // values compacted: 190 us, 195 in the other order, 185 without the votes)
+    const bool ok = wait_phase(&b_pre[k], (i / kSStages) & 1, polls);
+    const bool known = s_known[k];  // of use where every lane's wait ended
+    Sum run = s_pre[k];
+    for (int w = 0; w < warp; ++w) run += s_wsum[k][w];
+    if (__any_sync(kFull, !ok) || !known) {
       lost = true;
       if (lane == 0) atomicOr(&ctl->error, 1u);
     }
     if (!lost) {
-      Sum run = s_pre[k];
-      for (int w = 0; w < warp; ++w) run += s_wsum[k][w];
       op.finish(stage(k), (long long)tile[0] * kTileElems, run, warp, lane, carry[0], whole(tile[0]));
       // the warp's shared-memory writes before the bulk copy reads them (and
       // its reads before the stage's next bulk copy writes it)
