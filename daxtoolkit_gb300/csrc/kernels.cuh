@@ -267,8 +267,8 @@ constexpr int kAdjMinBlocks = 28;
 // time finding its grid, so sets of two waves of the larger blocks or more take
 // the larger count: 256 and 512 words a block with 6.3 of the larger blocks an SM
 // 37.9 and 38.3 us, 7.6 46.2 and 49.8, 11 51.4 and 50.4, 14.5 70 and 65, 19 87 and
-// 82, 46 181 and 166.  (Four blocks an SM instead of three: 32 grids of 45 M
-// points 72 -> 54 us.)
+// 82, 46 181 and 166.  (Four blocks an SM instead of three, with 24 bytes
+// spilled: 32 grids of 45 M points 72 -> 54 us.)
 constexpr int kEdgeWordsMost = 512, kEdgeWordsLeast = 256;
 
 struct MarchTiles {

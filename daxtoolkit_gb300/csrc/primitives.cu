@@ -837,7 +837,9 @@ constexpr int kSortWarps = kSortThreads / 32;
 // them, in different phases, share an SM: three of 4-byte keys with up to one
 // word of values, two otherwise (by registers and shared memory).  100 M int32
 // pairs: 2.14 ms with three of 384 threads, the same with two of 512, 2.36 with
-// two of 384; 30 M int64 pairs: 1.72, 2.18 (one block fits) and 1.72 ms.
+// two of 384; 30 M int64 pairs: 1.72, 2.18 (one block fits) and 1.72 ms.  (At
+// three blocks the form with one word of values spills 32 bytes, at two those
+// with three and four words 8 to 16.)
 constexpr int kSweepThreads = 384;
 constexpr int kSweepTile = kSweepThreads * kSortItems;
 constexpr int kSweepWarps = kSweepThreads / 32;

@@ -59,7 +59,7 @@ __device__ __forceinline__ uint2 plane_pairs(const uint32_t* __restrict__ bits, 
 // written where a point is used.  (Kept masks and used masks in two passes, four
 // words a lane: from the classification's end to the scan's 40 us at 512^3, 16
 // at 200 x 180 x 150, 17 at 60^3; now 34, 10 and 11, and with two blocks an SM
-// in place of four 39, 9 and 11.)
+// in place of four, which spill 12 bytes, 39, 9 and 11.)
 constexpr int kThrThreads = 512;
 __global__ void __launch_bounds__(kThrThreads, 4)
     k_thr_words(Grid g, const uint32_t* __restrict__ bits, uint32_t* __restrict__ kept,
